@@ -62,16 +62,12 @@ struct drpt_index {
   int32_t *csc_col = nullptr, *csc_row = nullptr;
   float *csc_val = nullptr;
   int ncols_r = 0;
+  int max_leaf = 0;
   __nv_bfloat16 *w1b = nullptr;
   float *b1 = nullptr, *w2 = nullptr, *b2 = nullptr, *c = nullptr, *inv_sigma = nullptr;
-  // query scratch, grown on demand
-  int64_t cap = 0;
-  float *Pq = nullptr;
-  int32_t *leaf = nullptr, *qi = nullptr;
-  float *qd = nullptr;
-  void *qx = nullptr;
-  __nv_bfloat16 *qxb = nullptr;
-  int *err = nullptr;
+  // query scratch, one allocation grown on demand
+  uint8_t *scratch = nullptr;
+  size_t scratch_bytes = 0;
 };
 
 namespace drpt {
@@ -1045,6 +1041,8 @@ drpt_status run_mixed(drpt_ctx *c, const drpt_build_desc *desc, const void *X, i
     DRPT_TRY(dev_copy((uint8_t **)&keep->X, X, (size_t)n * d * esz, s));
     DRPT_TRY(dev_copy(&keep->order, order, (size_t)T * n, s));
     DRPT_TRY(dev_copy(&keep->goff, goff, (size_t)T * (nleaf + 1), s));
+    std::vector<int32_t> h((size_t)T * (nleaf + 1));
+    DRPT_CUDA(cudaMemcpyAsync(h.data(), goff, h.size() * 4, cudaMemcpyDeviceToHost, s));
     DRPT_TRY(dev_copy(&keep->medians, medians, (size_t)T * std::max(nleaf - 1, 1), s));
     keep->ncols_r = (int)cols.size();
     if (!cols.empty()) {
@@ -1075,6 +1073,11 @@ drpt_status run_mixed(drpt_ctx *c, const drpt_build_desc *desc, const void *X, i
       DRPT_TRY(dev_copy(&keep->inv_sigma, is, 1, s));
     }
     DRPT_CUDA(cudaStreamSynchronize(s));
+    for (int t = 0; t < T; ++t)
+      for (int j = 0; j < nleaf; ++j) {
+        const int32_t *o = h.data() + (size_t)t * (nleaf + 1) + j;
+        keep->max_leaf = std::max(keep->max_leaf, o[1] - o[0]);
+      }
   }
   if (stats) {
     std::memset(stats, 0, sizeof(*stats));
@@ -1978,8 +1981,7 @@ static void index_free(drpt_index *x) {
   if (!x) return;
   cudaSetDevice(x->device);
   void *ptrs[] = {x->X, x->order, x->goff, x->medians, x->csc_col, x->csc_row, x->csc_val,
-                  x->w1b, x->b1, x->w2, x->b2, x->c, x->inv_sigma, x->Pq, x->leaf, x->qi,
-                  x->qd, x->qx, x->qxb, x->err};
+                  x->w1b, x->b1, x->w2, x->b2, x->c, x->inv_sigma, x->scratch};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   delete x;
@@ -2007,6 +2009,80 @@ drpt_status drpt_index_build(drpt_ctx *c, const drpt_build_desc *desc, const voi
 
 void drpt_index_destroy(drpt_index *index) { index_free(index); }
 
+// Entries of the candidate lists held at a time (8 bytes each: 512 MiB).
+static constexpr int64_t kQueryEntries = (int64_t)64 << 20;
+
+// One block of queries, stream-ordered.  `first`: clears the error flag of the
+// inference kernel, which later blocks of the call add to.
+static drpt_status query_block(drpt_index *x, const void *queries, int64_t nq, int k,
+                               int on_device, bool first, int32_t *out_idx, float *out_dist,
+                               int **err_out, cudaStream_t s) {
+  const int d = x->d, T = x->T, cols = T * (x->gd - 1);
+  const size_t esz = x->dtype == DRPT_DTYPE_U8 ? 1 : 4, pairs = (size_t)nq * T;
+  const bool aligned = !on_device || (uintptr_t)queries % (4 * esz) == 0;
+  const QueryPlan p = query_plan(nq, T, x->nleaf, x->max_leaf, k, aligned);
+  // the block's buffers, laid out in one allocation (16-byte aligned parts)
+  size_t total = 0;
+  auto part = [&](size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t o_err = part(4), o_P = part((size_t)cols * nq * 4), o_leaf = part(pairs * 4);
+  const size_t o_ci = part((size_t)p.entries * 4), o_cd = part((size_t)p.entries * 4);
+  const size_t o_cnt = part((size_t)p.buckets * 4), o_off = part((size_t)p.buckets * 4);
+  const size_t o_items = part((size_t)p.items * sizeof(int4)), o_nit = part(4);
+  const size_t o_rank = part(p.qt ? pairs * 4 : 0), o_list = part(p.qt ? pairs * 4 : 0);
+  const size_t o_qi = part(on_device ? 0 : (size_t)nq * k * 4);
+  const size_t o_qd = part(on_device && out_dist ? 0 : (size_t)nq * k * 4);
+  const size_t o_qx = part(on_device ? 0 : (size_t)nq * d * esz);
+  const size_t o_qxb = part(x->Tl > 0 ? (size_t)nq * x->d_pad * 2 : 0);
+  if (total > x->scratch_bytes) {
+    if (x->scratch) DRPT_CUDA(cudaFree(x->scratch));
+    x->scratch = nullptr;
+    x->scratch_bytes = 0;
+    DRPT_CUDA(cudaMalloc((void **)&x->scratch, total));
+    x->scratch_bytes = total;
+  }
+  uint8_t *b = x->scratch;
+  const void *Q = queries;
+  if (!on_device) {
+    DRPT_CUDA(cudaMemcpyAsync(b + o_qx, queries, (size_t)nq * d * esz, cudaMemcpyHostToDevice, s));
+    Q = b + o_qx;
+  }
+  // the queries' split values: random columns, then the learned MLP outputs
+  float *P = (float *)(b + o_P);
+  if (x->ncols_r > 0) {
+    CscDev csc{x->csc_col, x->csc_row, x->csc_val, x->ncols_r};
+    DRPT_TRY(launch_project(Q, x->dtype, nq, d, csc, P, s));
+  }
+  if (x->Tl > 0) {
+    int *err = (int *)(b + o_err);
+    __nv_bfloat16 *xb = (__nv_bfloat16 *)(b + o_qxb);
+    if (first) DRPT_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+    DRPT_TRY(launch_standardise(Q, x->dtype, nq, d, x->d_pad, nullptr, x->c, x->inv_sigma, xb,
+                                nullptr, s));
+    DRPT_TRY(launch_mlp_infer(xb, nq, x->d_pad, x->w1b, x->Tl * (x->gd - 1), x->b1, x->w2, x->b2,
+                              P + (int64_t)x->ncols_r * nq, err, s));
+    *err_out = err;
+  }
+  int32_t *leaf = (int32_t *)(b + o_leaf);
+  DRPT_TRY(launch_descend(P, nq, T, x->gd, x->medians, leaf, s));
+  int32_t *oi = on_device ? out_idx : (int32_t *)(b + o_qi);
+  float *od = on_device && out_dist ? out_dist : (float *)(b + o_qd);
+  const QueryArgs a{x->X, x->dtype, d, x->n, Q, nq, T, x->order, x->goff, x->nleaf, leaf, k,
+                    (int32_t *)(b + o_ci), (float *)(b + o_cd), (int32_t *)(b + o_rank),
+                    (int32_t *)(b + o_cnt), (int32_t *)(b + o_off), (int4 *)(b + o_items),
+                    (int32_t *)(b + o_nit), (int32_t *)(b + o_list), oi, od};
+  DRPT_TRY(launch_query(a, p, s));
+  if (!on_device) {
+    DRPT_CUDA(cudaMemcpyAsync(out_idx, oi, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, s));
+    if (out_dist)
+      DRPT_CUDA(cudaMemcpyAsync(out_dist, od, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, s));
+  }
+  return DRPT_OK;
+}
+
 drpt_status drpt_index_query(drpt_index *x, const void *queries, int64_t nq, int32_t k,
                              int32_t on_device, int32_t *out_idx, float *out_dist, void *stream) {
   if (!x || !queries || !out_idx || nq <= 0 || k <= 0) return DRPT_ERR_INVALID_ARG;
@@ -2016,56 +2092,17 @@ drpt_status drpt_index_query(drpt_index *x, const void *queries, int64_t nq, int
   }
   DRPT_CUDA(cudaSetDevice(x->device));
   cudaStream_t s = (cudaStream_t)stream;
-  const int d = x->d, T = x->T, cols = T * (x->gd - 1);
+  // blocks of queries whose candidate lists stay within kQueryEntries
+  const int64_t most = std::max<int64_t>(1, kQueryEntries / ((int64_t)x->T * k));
   const size_t esz = x->dtype == DRPT_DTYPE_U8 ? 1 : 4;
-  if (nq > x->cap) {  // grow the query scratch
-    void **bufs[] = {(void **)&x->Pq, (void **)&x->leaf, (void **)&x->qi, (void **)&x->qd,
-                     (void **)&x->qx, (void **)&x->qxb, (void **)&x->err};
-    for (void **b : bufs)
-      if (*b) {
-        cudaFree(*b);
-        *b = nullptr;
-      }
-    x->cap = 0;
-    DRPT_CUDA(cudaMalloc((void **)&x->Pq, std::max<size_t>((size_t)cols * nq, 1) * 4));
-    DRPT_CUDA(cudaMalloc((void **)&x->leaf, (size_t)T * nq * 4));
-    DRPT_CUDA(cudaMalloc((void **)&x->qi, (size_t)32 * nq * 4));
-    DRPT_CUDA(cudaMalloc((void **)&x->qd, (size_t)32 * nq * 4));
-    DRPT_CUDA(cudaMalloc(&x->qx, (size_t)nq * d * esz));
-    if (x->Tl > 0) DRPT_CUDA(cudaMalloc((void **)&x->qxb, (size_t)nq * x->d_pad * 2));
-    DRPT_CUDA(cudaMalloc((void **)&x->err, sizeof(int)));
-    x->cap = nq;
-  }
-  const void *Q = queries;
-  if (!on_device) {
-    DRPT_CUDA(cudaMemcpyAsync(x->qx, queries, (size_t)nq * d * esz, cudaMemcpyHostToDevice, s));
-    Q = x->qx;
-  }
-  // the queries' split values: random columns, then the learned MLP outputs
-  if (x->ncols_r > 0) {
-    CscDev csc{x->csc_col, x->csc_row, x->csc_val, x->ncols_r};
-    DRPT_TRY(launch_project(Q, x->dtype, nq, d, csc, x->Pq, s));
-  }
-  if (x->Tl > 0) {
-    DRPT_CUDA(cudaMemsetAsync(x->err, 0, sizeof(int), s));
-    DRPT_TRY(launch_standardise(Q, x->dtype, nq, d, x->d_pad, nullptr, x->c, x->inv_sigma, x->qxb,
-                                nullptr, s));
-    DRPT_TRY(launch_mlp_infer(x->qxb, nq, x->d_pad, x->w1b, x->Tl * (x->gd - 1), x->b1, x->w2,
-                              x->b2, x->Pq + (int64_t)x->ncols_r * nq, x->err, s));
-  }
-  DRPT_TRY(launch_descend(x->Pq, nq, T, x->gd, x->medians, x->leaf, s));
-  int32_t *oi = on_device ? out_idx : x->qi;
-  float *od = on_device ? (out_dist ? out_dist : x->qd) : x->qd;
-  DRPT_TRY(launch_query(x->X, x->dtype, d, x->n, Q, nq, T, x->order, x->goff, x->nleaf, x->leaf,
-                        k, oi, od, s));
-  if (!on_device) {
-    DRPT_CUDA(cudaMemcpyAsync(out_idx, oi, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, s));
-    if (out_dist)
-      DRPT_CUDA(cudaMemcpyAsync(out_dist, od, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, s));
-  }
+  int *err = nullptr;
+  for (int64_t q0 = 0; q0 < nq; q0 += most)
+    DRPT_TRY(query_block(x, static_cast<const uint8_t *>(queries) + (size_t)q0 * x->d * esz,
+                         std::min(most, nq - q0), k, on_device, q0 == 0, out_idx + q0 * k,
+                         out_dist ? out_dist + q0 * k : nullptr, &err, s));
   if (x->Tl > 0) {
     int herr = 0;
-    DRPT_CUDA(cudaMemcpyAsync(&herr, x->err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    DRPT_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s));
     DRPT_CUDA(cudaStreamSynchronize(s));
     if (herr) {
       set_error("a bounded wait in the split-MLP inference kernel gave up");

@@ -6,15 +6,18 @@
 //                 query's projected values and the stored node medians,
 //                 `value <= median` going left as in the build
 //                 (drpt_global.cpp:308); ends at a global leaf
-//   Q2 k_query    per query one warp: the members of its leaf in every tree,
-//                 32 at a time (one per lane), exact FP32 distances
-//                 (sequential fused multiply-adds over the dimensions,
-//                 square root), a warp-wide list of the k best by
-//                 (distance, id): a batch that beats the k-th is sorted
-//                 with a shuffle bitonic network and merged into the list;
-//                 members already in the list are skipped, so a point found
-//                 in several trees counts once
+//   Q2            exact FP32 distances (sequential fused multiply-adds over
+//                 the dimensions, square root) of the members of each query's
+//                 leaf in every tree, and the k best of them by (distance,
+//                 id): k_query_few reads a leaf for each query, k_query_tile
+//                 once for all queries that fall in it
+//   Q3            the trees' lists merged (a point found in several trees
+//                 counts once): k_query_join, or the builds' cross-tree merge
+#include <algorithm>
+#include <type_traits>
+
 #include "kernels.cuh"
+#include "sm100.cuh"
 
 namespace drpt {
 namespace {
@@ -70,101 +73,430 @@ __device__ __forceinline__ float4 ld4<uint8_t>(const uint8_t *p) {
   return make_float4(v.x, v.y, v.z, v.w);
 }
 
-template <typename T, typename TQ>
-__global__ void __launch_bounds__(256) k_query(const T *__restrict__ X, int d, int64_t n,
-                                               const TQ *__restrict__ Qx, int64_t nq, int T_,
-                                               const int32_t *__restrict__ order,
-                                               const int32_t *__restrict__ goff, int nleaf,
-                                               const int32_t *__restrict__ leaf, int k,
-                                               int32_t *__restrict__ oi, float *__restrict__ od) {
-  extern __shared__ float qs[];  // 8 warps x d query values
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t q = (int64_t)blockIdx.x * 8 + warp;
-  if (q >= nq) return;  // warp-uniform; no block barrier below
-  float *qv = qs + (int64_t)warp * d;
-  for (int c = lane; c < d; c += 32) qv[c] = (float)Qx[q * d + c];
-  __syncwarp();
-  const float inf = __int_as_float(0x7f800000);
-  float ld = inf;  // the list: lane j holds the j-th best (j < 32)
-  int32_t li = -1;
-  for (int t = 0; t < T_; ++t) {
-    const int lf = leaf[q * T_ + t];
-    const int32_t *go = goff + (int64_t)t * (nleaf + 1);
-    const int32_t lo = go[lf], hi = go[lf + 1];
-    const int32_t *ord = order + (int64_t)t * n;
-    for (int32_t base = lo; base < hi; base += 32) {
-      const int32_t pos = base + lane;
-      const int32_t p = pos < hi ? __ldg(ord + pos) : -1;
-      float dist = inf;
-      if (p >= 0) {
-        const T *row = X + (int64_t)p * d;
-        float acc = 0.0f;
-        for (int c = 0; c < d; c += 4) {  // d % 4 == 0
-          const float4 x = ld4<T>(row + c);
-          const float4 y = *reinterpret_cast<const float4 *>(qv + c);
-          float df = x.x - y.x;
-          acc = fmaf(df, df, acc);
-          df = x.y - y.y;
-          acc = fmaf(df, df, acc);
-          df = x.z - y.z;
-          acc = fmaf(df, df, acc);
-          df = x.w - y.w;
-          acc = fmaf(df, df, acc);
-        }
-        dist = sqrtf(acc);
-      }
-      // skip members the list already holds, and those that cannot enter it
-      const float kd = __shfl_sync(kFull, ld, k - 1);
-      const int32_t ki = __shfl_sync(kFull, li, k - 1);
-      // every lane takes part in every shuffle (a full-mask shuffle that some
-      // lanes skip never completes)
-      bool dup = false;
-#pragma unroll 8
-      for (int j = 0; j < 32; ++j) {
-        const int32_t lj = __shfl_sync(kFull, li, j);
-        dup |= (p >= 0 && lj == p);
-      }
-      int32_t cid = p;
-      if (dup || p < 0 || !qbefore(dist, p, kd, ki)) {
-        dist = inf;
-        cid = -1;
-      }
-      if (!__any_sync(kFull, cid >= 0)) continue;
-      warp_sort32(dist, cid, lane);
-      // the 32 smallest of list and batch: min of the list and the reversed
-      // batch is bitonic; a bitonic clean sorts it
-      const float rd = __shfl_sync(kFull, dist, 31 - lane);
-      const int32_t ri = __shfl_sync(kFull, cid, 31 - lane);
-      if (qbefore(rd, ri, ld, li)) {
-        ld = rd;
-        li = ri;
-      }
+// L (sorted over the lanes) <- the 32 smallest of L and a sorted batch: the
+// minimum of L and the reversed batch is bitonic; a bitonic clean sorts it.
+__device__ __forceinline__ void warp_merge32(float &ld, int32_t &li, float d, int32_t id,
+                                             int lane) {
+  const float rd = __shfl_sync(kFull, d, 31 - lane);
+  const int32_t ri = __shfl_sync(kFull, id, 31 - lane);
+  if (qbefore(rd, ri, ld, li)) {
+    ld = rd;
+    li = ri;
+  }
 #pragma unroll
-      for (int stride = 16; stride > 0; stride >>= 1) {
-        const float odv = __shfl_xor_sync(kFull, ld, stride);
-        const int32_t oiv = __shfl_xor_sync(kFull, li, stride);
-        const bool lower = (lane & stride) == 0;
-        const bool mine_first = qbefore(ld, li, odv, oiv);
-        if (lower != mine_first) {
-          ld = odv;
-          li = oiv;
-        }
-      }
+  for (int stride = 16; stride > 0; stride >>= 1) {
+    const float od = __shfl_xor_sync(kFull, ld, stride);
+    const int32_t oi = __shfl_xor_sync(kFull, li, stride);
+    const bool lower = (lane & stride) == 0;
+    const bool mine_first = qbefore(ld, li, od, oi);
+    if (lower != mine_first) {
+      ld = od;
+      li = oi;
     }
   }
+}
+
+// The warp's sorted list <- its 32 smallest with this lane's candidate
+// (id < 0: none).  Only candidates before the list's k-th entry enter; a few
+// are inserted one by one (a ballot and a shift each), more are sorted and
+// merged as a batch.  Every lane takes part in every shuffle.
+__device__ __forceinline__ void warp_take(float &ld, int32_t &li, float d, int32_t id, int k,
+                                          int lane) {
+  const float kd = __shfl_sync(kFull, ld, k - 1);
+  const int32_t ki = __shfl_sync(kFull, li, k - 1);
+  const bool pass = id >= 0 && qbefore(d, id, kd, ki);
+  unsigned m = __ballot_sync(kFull, pass);
+  if (m == 0) return;
+  if (__popc(m) > 5) {
+    float bd = pass ? d : __int_as_float(0x7f800000);
+    int32_t bi = pass ? id : -1;
+    warp_sort32(bd, bi, lane);
+    warp_merge32(ld, li, bd, bi, lane);
+    return;
+  }
+  do {
+    const int src = __ffs(m) - 1;
+    m &= m - 1;
+    const float v = __shfl_sync(kFull, d, src);
+    const int32_t i = __shfl_sync(kFull, id, src);
+    const int at = __popc(__ballot_sync(kFull, qbefore(ld, li, v, i)));
+    const float ud = __shfl_up_sync(kFull, ld, 1);
+    const int32_t ui = __shfl_up_sync(kFull, li, 1);
+    if (lane == at) {
+      ld = v;
+      li = i;
+    } else if (lane > at) {
+      ld = ud;
+      li = ui;
+    }
+  } while (m);
+}
+
+// Q2a, few queries: block (e, s) takes share s of the S shares of the
+// members of query e / T's leaf in tree e % T; warps take 32 members at a
+// time, a lane each.  Latency bounds it (one query: a few thousand members),
+// so the members spread over T * S blocks of eight warps and a lane keeps
+// kBurst 16-byte pieces of its row in flight; a whole leaf per query on one
+// warp took 911 us for one query of 6 trees with 1,024-point leaves.
+constexpr int kFewWarps = 8;
+template <typename T>
+__global__ void __launch_bounds__(32 * kFewWarps) k_query_few(
+    const T *__restrict__ X, int d, int64_t n, const T *__restrict__ Qx, int T_, int S,
+    const int32_t *__restrict__ order, const int32_t *__restrict__ goff, int nleaf,
+    const int32_t *__restrict__ leaf, int k, int32_t *__restrict__ ci, float *__restrict__ cd) {
+  constexpr int kBurst = 8;
+  extern __shared__ __align__(16) float qv[];  // the query's d values
+  __shared__ float sd[kFewWarps][32];
+  __shared__ int32_t si[kFewWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t e = blockIdx.x / S;
+  const int s = (int)(blockIdx.x - e * S);
+  const int64_t q = e / T_;
+  const int t = (int)(e - q * T_);
+  for (int c = threadIdx.x; c < d; c += blockDim.x) qv[c] = (float)Qx[q * d + c];
+  const int lf = __ldg(leaf + e);
+  const int32_t *go = goff + (int64_t)t * (nleaf + 1);
+  const int32_t lo0 = __ldg(go + lf), m = __ldg(go + lf + 1) - lo0;
+  const int32_t per = ((m + S - 1) / S + 31) & ~31;
+  const int32_t lo = lo0 + min(s * per, m), hi = lo0 + min((s + 1) * per, m);
+  const int32_t *ord = order + (int64_t)t * n;
+  __syncthreads();
+  const float inf = __int_as_float(0x7f800000);
+  float ld = inf;  // the list: lane j holds the j-th best
+  int32_t li = -1;
+  for (int32_t base = lo + 32 * warp; base < hi; base += 32 * kFewWarps) {
+    const int32_t pos = base + lane;
+    const int32_t p = pos < hi ? __ldg(ord + pos) : -1;
+    const T *row = X + (int64_t)max(p, 0) * d;
+    float acc = 0.0f;
+    for (int c0 = 0; c0 < d; c0 += 4 * kBurst) {  // d % 4 == 0
+      float4 x[kBurst];
+#pragma unroll
+      for (int i = 0; i < kBurst; ++i)
+        if (c0 + 4 * i < d) x[i] = ld4<T>(row + c0 + 4 * i);
+#pragma unroll
+      for (int i = 0; i < kBurst; ++i)
+        if (c0 + 4 * i < d) {
+          const float4 y = *reinterpret_cast<const float4 *>(qv + c0 + 4 * i);
+          float df = x[i].x - y.x;
+          acc = fmaf(df, df, acc);
+          df = x[i].y - y.y;
+          acc = fmaf(df, df, acc);
+          df = x[i].z - y.z;
+          acc = fmaf(df, df, acc);
+          df = x[i].w - y.w;
+          acc = fmaf(df, df, acc);
+        }
+    }
+    warp_take(ld, li, sqrtf(acc), p, k, lane);
+  }
+  sd[warp][lane] = ld;
+  si[warp][lane] = li;
+  __syncthreads();
+  if (warp != 0) return;
+  for (int w = 1; w < kFewWarps; ++w) warp_merge32(ld, li, sd[w][lane], si[w][lane], lane);
+  if (lane < k) {
+    ci[(int64_t)blockIdx.x * k + lane] = li;
+    cd[(int64_t)blockIdx.x * k + lane] = ld;
+  }
+}
+
+// Q3, few queries: one block per query merges its `lists` sorted lists of k
+// entries (the same member from two trees carries the same distance bits, so
+// it counts once); warps take lists in turn, warp 0 joins the warps' lists.
+__device__ __forceinline__ void warp_join(float &ld, int32_t &li, float d, int32_t id, int k,
+                                          int lane) {
+  bool dup = false;
+  for (int j = 0; j < k; ++j) dup |= __shfl_sync(kFull, li, j) == id;
+  if (dup || lane >= k) id = -1;
+  warp_take(ld, li, d, id, k, lane);
+}
+
+__global__ void __launch_bounds__(32 * kFewWarps) k_query_join(const int32_t *__restrict__ ci,
+                                                               const float *__restrict__ cd,
+                                                               int lists, int k,
+                                                               int32_t *__restrict__ oi,
+                                                               float *__restrict__ od) {
+  __shared__ float sd[kFewWarps][32];
+  __shared__ int32_t si[kFewWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t q = blockIdx.x;
+  const float inf = __int_as_float(0x7f800000);
+  float ld = inf;
+  int32_t li = -1;
+  for (int l = warp; l < lists; l += kFewWarps) {
+    const int64_t o = (q * lists + l) * k + lane;
+    warp_join(ld, li, lane < k ? __ldg(cd + o) : inf, lane < k ? __ldg(ci + o) : -1, k, lane);
+  }
+  sd[warp][lane] = ld;
+  si[warp][lane] = li;
+  __syncthreads();
+  if (warp != 0) return;
+  for (int w = 1; w < min(kFewWarps, lists); ++w)
+    warp_join(ld, li, sd[w][lane], si[w][lane], k, lane);
   if (lane < k) {
     oi[q * k + lane] = li;
     od[q * k + lane] = li >= 0 ? ld : inf;
   }
 }
 
-template <typename T, typename TQ>
-void query_t(const void *X, int d, int64_t n, const void *Qx, int64_t nq, int T_,
-             const int32_t *order, const int32_t *goff, int nleaf, const int32_t *leaf, int k,
-             int32_t *oi, float *od, cudaStream_t s) {
-  const size_t smem = (size_t)8 * d * sizeof(float);
-  k_query<T, TQ><<<(unsigned)ceil_div(nq, 8), 256, smem, s>>>(
-      (const T *)X, d, n, (const TQ *)Qx, nq, T_, order, goff, nleaf, leaf, k, oi, od);
+// Many queries: the (query, tree) pairs grouped by leaf, so that a leaf's
+// rows are staged once for up to QT queries.
+//   k_query_count  pairs per (tree, leaf) and each pair's place among them
+//   k_query_plan   leaf offsets in the grouped list, items of <= QT queries
+//   k_query_fill   the grouped list
+__global__ void k_query_count(const int32_t *__restrict__ leaf, int64_t nq, int T_, int nleaf,
+                              int32_t *__restrict__ cnt, int32_t *__restrict__ rank) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nq * T_) return;
+  rank[e] = atomicAdd(cnt + (int64_t)(e % T_) * nleaf + leaf[e], 1);
+}
+
+__global__ void __launch_bounds__(1024) k_query_plan(const int32_t *__restrict__ cnt, int B,
+                                                     int qt, int32_t *__restrict__ off,
+                                                     int4 *__restrict__ items,
+                                                     int32_t *__restrict__ n_items) {
+  __shared__ int tot[2][32];
+  const int per = (B + 1023) / 1024;
+  const int b0 = threadIdx.x * per, b1 = min(b0 + per, B);
+  int c = 0, it = 0;
+  for (int b = b0; b < b1; ++b) {
+    c += cnt[b];
+    it += (cnt[b] + qt - 1) / qt;
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int xc = c, xi = it;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int yc = __shfl_up_sync(kFull, xc, o), yi = __shfl_up_sync(kFull, xi, o);
+    if (lane >= o) {
+      xc += yc;
+      xi += yi;
+    }
+  }
+  if (lane == 31) {
+    tot[0][w] = xc;
+    tot[1][w] = xi;
+  }
+  __syncthreads();
+  if (w < 2) {
+    int v = tot[w][lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(kFull, v, o);
+      if (lane >= o) v += y;
+    }
+    tot[w][lane] = v;
+  }
+  __syncthreads();
+  int oc = xc - c + (w > 0 ? tot[0][w - 1] : 0), oi = xi - it + (w > 0 ? tot[1][w - 1] : 0);
+  for (int b = b0; b < b1; ++b) {
+    off[b] = oc;
+    for (int q = 0; q < cnt[b]; q += qt) items[oi++] = make_int4(b, oc + q, min(qt, cnt[b] - q), 0);
+    oc += cnt[b];
+  }
+  if (threadIdx.x == 1023) *n_items = oi;
+}
+
+__global__ void k_query_fill(const int32_t *__restrict__ leaf, const int32_t *__restrict__ rank,
+                             const int32_t *__restrict__ off, int64_t nq, int T_, int nleaf,
+                             int32_t *__restrict__ list) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nq * T_) return;
+  list[off[(int64_t)(e % T_) * nleaf + leaf[e]] + rank[e]] = (int32_t)(e / T_);
+}
+
+// Q2b: one item (<= QT queries of one leaf) against every kMT-member tile of
+// the leaf.  Members and queries are staged in kKc-dimension chunks, dimension
+// major, through two shared buffers (the next chunk is in registers while the
+// current one is used); thread (ty, tx) owns queries ty + 16 i and members
+// 4 tx + j, 64 + 4 tx + j: a packed subtraction and a packed multiply-add take
+// two members at once, each pair's sum running over the dimensions in order as
+// in k_query_few.  Then eight lanes' worth of selection: warp w keeps the
+// lists of queries w QT/8 .. in its lanes.  FP32 issue bounds it: two
+// operations per dimension and pair.  QT = 64 serves buckets that fill it;
+// QT = 16 smaller ones, where 64 would mostly compute padding.
+constexpr int kMT = 128, kKc = 32, kQThreads = 256;
+constexpr int kSPitch = kMT + 4;
+template <int QT>
+constexpr size_t query_smem() {
+  return sizeof(float) * (2 * kKc * kMT + 2 * kKc * QT * 2 + QT * kSPitch) +
+         sizeof(int32_t) * (kMT + QT);
+}
+
+template <typename T, int QT>
+__global__ void __launch_bounds__(kQThreads, 2) k_query_tile(
+    const T *__restrict__ X, int d, int64_t n, const T *__restrict__ Qx, int T_,
+    const int32_t *__restrict__ order, const int32_t *__restrict__ goff, int nleaf,
+    const int4 *__restrict__ items, const int32_t *__restrict__ n_items,
+    const int32_t *__restrict__ list, int k, int32_t *__restrict__ ci, float *__restrict__ cd) {
+  constexpr int QPT = QT / 16;   // queries per thread
+  constexpr int QPW = QT / 8;    // queries per warp in the selection
+  constexpr int QG = QT * kKc / 4 / kQThreads > 0 ? QT * kKc / 4 / kQThreads : 1;  // query quads
+  extern __shared__ __align__(16) float sm[];
+  float *Ms = sm;                               // [2][kKc][kMT]
+  float *Qs = Ms + 2 * kKc * kMT;               // [2][kKc][QT][2]: -y twice
+  float *St = Qs + 2 * kKc * QT * 2;            // [QT][kSPitch]
+  int32_t *cid = reinterpret_cast<int32_t *>(St + QT * kSPitch);  // kMT
+  int32_t *qid = cid + kMT;                     // QT
+  if ((int)blockIdx.x >= *n_items) return;
+  const int4 item = items[blockIdx.x];
+  const int t = item.x / nleaf, lf = item.x - t * nleaf, nqi = item.z;
+  const int32_t *go = goff + (int64_t)t * (nleaf + 1);
+  const int32_t lo = __ldg(go + lf), m = __ldg(go + lf + 1) - lo;
+  const int32_t *ord = order + (int64_t)t * n + lo;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int warp = tid >> 5, lane = tid & 31;
+  if (tid < QT) qid[tid] = tid < nqi ? __ldg(list + item.y + tid) : -1;
+  __syncthreads();
+  // staging: member sr, 16 dimensions from sk; query quads (row, 4 dimensions)
+  const int sr = tid & (kMT - 1), sk = (tid >> 7) * 16;
+  float4 pm[4], pq[QG];
+  auto member = [&](int m0) { return m0 + sr < m ? __ldg(ord + m0 + sr) : -1; };
+  auto fetch = [&](int32_t row, int k0) {
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = k0 + sk + 4 * i;
+      pm[i] = row >= 0 && c < d ? ld4<T>(X + (int64_t)row * d + c) : z;
+    }
+#pragma unroll
+    for (int i = 0; i < QG; ++i) {
+      const int g = tid + i * kQThreads, r = g % QT, c = k0 + 4 * (g / QT);
+      pq[i] = z;
+      if (g < QT * (kKc / 4) && qid[r] >= 0 && c < d) pq[i] = ld4<T>(Qx + (int64_t)qid[r] * d + c);
+    }
+  };
+  auto store = [&](int b) {
+    float *M = Ms + b * kKc * kMT;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      M[(sk + 4 * i) * kMT + sr] = pm[i].x;
+      M[(sk + 4 * i + 1) * kMT + sr] = pm[i].y;
+      M[(sk + 4 * i + 2) * kMT + sr] = pm[i].z;
+      M[(sk + 4 * i + 3) * kMT + sr] = pm[i].w;
+    }
+#pragma unroll
+    for (int i = 0; i < QG; ++i) {
+      const int g = tid + i * kQThreads, r = g % QT, c = 4 * (g / QT);
+      if (g < QT * (kKc / 4)) {
+        float2 *Q = reinterpret_cast<float2 *>(Qs) + (b * kKc + c) * QT + r;
+        Q[0] = make_float2(-pq[i].x, -pq[i].x);
+        Q[QT] = make_float2(-pq[i].y, -pq[i].y);
+        Q[2 * QT] = make_float2(-pq[i].z, -pq[i].z);
+        Q[3 * QT] = make_float2(-pq[i].w, -pq[i].w);
+      }
+    }
+  };
+  const float inf = __int_as_float(0x7f800000);
+  float ld[QPW];
+  int32_t li[QPW];
+#pragma unroll
+  for (int i = 0; i < QPW; ++i) {
+    ld[i] = inf;
+    li[i] = -1;
+  }
+  int32_t row = member(0);
+  fetch(row, 0);
+  for (int m0 = 0; m0 < m; m0 += kMT) {
+    const int32_t next = member(m0 + kMT);
+    float2 acc[QPT][4];
+#pragma unroll
+    for (int i = 0; i < QPT; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+    store(0);
+    __syncthreads();  // chunk 0 stored; the previous tile's selection is done
+    if (tid < kMT) cid[tid] = row;
+    int cur = 0;
+    for (int k0 = 0; k0 < d; k0 += kKc, cur ^= 1) {
+      const bool more = k0 + kKc < d;
+      if (more) fetch(row, k0 + kKc);
+      else if (m0 + kMT < m) fetch(next, 0);
+      const float *M = Ms + cur * kKc * kMT;
+      const float2 *Q = reinterpret_cast<const float2 *>(Qs) + cur * kKc * QT;
+#pragma unroll 8
+      for (int kk = 0; kk < kKc; ++kk) {
+        const float4 a = *reinterpret_cast<const float4 *>(M + kk * kMT + 4 * tx);
+        const float4 b = *reinterpret_cast<const float4 *>(M + kk * kMT + 64 + 4 * tx);
+        const float2 x[4] = {make_float2(a.x, a.y), make_float2(a.z, a.w),
+                             make_float2(b.x, b.y), make_float2(b.z, b.w)};
+#pragma unroll
+        for (int i = 0; i < QPT; ++i) {
+          const float2 y = Q[kk * QT + ty + 16 * i];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 df = sm100::add2(x[j], y);
+            acc[i][j] = sm100::fma2(df, df, acc[i][j]);
+          }
+        }
+      }
+      // the other buffer was last read before the barrier that ended the
+      // previous chunk
+      if (more) {
+        store(cur ^ 1);
+        __syncthreads();
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < QPT; ++i) {
+      float *s = St + (ty + 16 * i) * kSPitch;
+      *reinterpret_cast<float4 *>(s + 4 * tx) =
+          make_float4(sqrtf(acc[i][0].x), sqrtf(acc[i][0].y), sqrtf(acc[i][1].x),
+                      sqrtf(acc[i][1].y));
+      *reinterpret_cast<float4 *>(s + 64 + 4 * tx) =
+          make_float4(sqrtf(acc[i][2].x), sqrtf(acc[i][2].y), sqrtf(acc[i][3].x),
+                      sqrtf(acc[i][3].y));
+    }
+    __syncthreads();  // scores and ids stored; every chunk read
+#pragma unroll
+    for (int i = 0; i < QPW; ++i) {
+      const int q = warp * QPW + i;
+      if (q < nqi) {  // warp-uniform
+#pragma unroll
+        for (int h = 0; h < kMT / 32; ++h)
+          warp_take(ld[i], li[i], St[q * kSPitch + 32 * h + lane], cid[32 * h + lane], k, lane);
+      }
+    }
+    row = next;
+  }
+#pragma unroll
+  for (int i = 0; i < QPW; ++i) {
+    const int q = warp * QPW + i;
+    if (q < nqi && lane < k) {
+      const int64_t o = ((int64_t)qid[q] * T_ + t) * k + lane;
+      ci[o] = li[i];
+      cd[o] = ld[i];
+    }
+  }
+}
+
+template <typename T, int QT>
+drpt_status query_tile(const QueryArgs &a, unsigned max_items, cudaStream_t s) {
+  constexpr size_t smem = query_smem<QT>();
+  DRPT_CUDA(cudaFuncSetAttribute(k_query_tile<T, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem));
+  k_query_tile<T, QT><<<max_items, kQThreads, smem, s>>>(
+      (const T *)a.X, a.d, a.n, (const T *)a.Q, a.T, a.order, a.goff, a.nleaf, a.items, a.n_items,
+      a.list, a.k, a.ci, a.cd);
+  DRPT_LAUNCH_CHECK();
+  return DRPT_OK;
+}
+
+// Queries per item of the grouped form; 0: the few-queries form.  The grouped
+// form stages a leaf once for the queries that fall in it (nq / nleaf on
+// average), the other one reads it for each query.
+constexpr int kQueryWide = 24, kQueryGroup = 2;
+int query_group(int64_t nq, int nleaf) {
+  const int64_t per = nq / nleaf;
+  return per >= kQueryWide ? 64 : (per >= kQueryGroup ? 16 : 0);
+}
+
+// Shares that the few-queries form cuts a leaf into: until the pairs fill the
+// SMs, but no share below the block's 256 members.
+int query_shares(int64_t pairs, int max_leaf) {
+  const int most = (int)ceil_div(std::max(max_leaf, 1), 32 * kFewWarps);
+  return (int)std::max<int64_t>(1, std::min<int64_t>(most, 8 * 148 / std::max<int64_t>(pairs, 1)));
 }
 
 }  // namespace
@@ -177,20 +509,66 @@ drpt_status launch_descend(const float *Pq, int64_t nq, int T, int gd, const flo
   return DRPT_OK;
 }
 
-drpt_status launch_query(const void *X, int dtype, int d, int64_t n, const void *Qx, int64_t nq,
-                         int T, const int32_t *order, const int32_t *goff, int nleaf,
-                         const int32_t *leaf, int k, int32_t *oi, float *od, cudaStream_t s) {
-  if (nq <= 0) return DRPT_OK;
-  if (k <= 0 || k > 32 || d % 4 != 0 || d > 1024) {
-    set_error("queries: k in [1, 32] and d %% 4 == 0, d <= 1024 (got k %d, d %d)", k, d);
+// `aligned`: the query rows can be read in 16-byte (u8: 4-byte) pieces, as the
+// grouped form does.
+QueryPlan query_plan(int64_t nq, int T, int nleaf, int max_leaf, int k, bool aligned) {
+  QueryPlan p{};
+  p.qt = aligned ? query_group(nq, nleaf) : 0;
+  const int64_t pairs = nq * T;
+  if (p.qt == 0) {
+    p.shares = query_shares(pairs, max_leaf);
+    p.lists = pairs * p.shares;
+  } else {
+    p.shares = 1;
+    p.lists = pairs;
+    p.buckets = (int64_t)T * nleaf;
+    p.items = ceil_div(pairs, p.qt) + std::min<int64_t>(p.buckets, pairs);
+  }
+  p.entries = p.lists * k;
+  return p;
+}
+
+drpt_status launch_query(const QueryArgs &a, const QueryPlan &p, cudaStream_t s) {
+  if (a.nq <= 0) return DRPT_OK;
+  if (a.k <= 0 || a.k > 32 || a.d % 4 != 0 || a.d > 1024) {
+    set_error("queries: k in [1, 32] and d %% 4 == 0, d <= 1024 (got k %d, d %d)", a.k, a.d);
     return DRPT_ERR_UNSUPPORTED;
   }
-  if (dtype == DRPT_DTYPE_U8)
-    query_t<uint8_t, uint8_t>(X, d, n, Qx, nq, T, order, goff, nleaf, leaf, k, oi, od, s);
-  else
-    query_t<float, float>(X, d, n, Qx, nq, T, order, goff, nleaf, leaf, k, oi, od, s);
-  DRPT_LAUNCH_CHECK();
-  return DRPT_OK;
+  const bool u8 = a.dtype == DRPT_DTYPE_U8;
+  if (p.qt == 0) {
+    if (p.lists > 0x7fffffff) {
+      set_error("queries: %lld (query, tree) pairs in one launch", (long long)p.lists);
+      return DRPT_ERR_UNSUPPORTED;
+    }
+    auto few = [&](auto *X, auto *Q) {
+      using E = std::remove_const_t<std::remove_pointer_t<decltype(X)>>;
+      k_query_few<E><<<(unsigned)p.lists, 32 * kFewWarps, a.d * sizeof(float), s>>>(
+          X, a.d, a.n, Q, a.T, p.shares, a.order, a.goff, a.nleaf, a.leaf, a.k, a.ci, a.cd);
+    };
+    if (u8) few((const uint8_t *)a.X, (const uint8_t *)a.Q);
+    else few((const float *)a.X, (const float *)a.Q);
+    DRPT_LAUNCH_CHECK();
+    if (p.shares > 1) {
+      k_query_join<<<(unsigned)a.nq, 32 * kFewWarps, 0, s>>>(a.ci, a.cd, a.T * p.shares, a.k, a.oi,
+                                                             a.od);
+      DRPT_LAUNCH_CHECK();
+      return DRPT_OK;
+    }
+  } else {
+    const int64_t pairs = a.nq * a.T;
+    const unsigned grid = (unsigned)ceil_div(pairs, 256);
+    DRPT_CUDA(cudaMemsetAsync(a.cnt, 0, (size_t)p.buckets * 4, s));
+    k_query_count<<<grid, 256, 0, s>>>(a.leaf, a.nq, a.T, a.nleaf, a.cnt, a.rank);
+    k_query_plan<<<1, 1024, 0, s>>>(a.cnt, (int)p.buckets, p.qt, a.off, a.items, a.n_items);
+    k_query_fill<<<grid, 256, 0, s>>>(a.leaf, a.rank, a.off, a.nq, a.T, a.nleaf, a.list);
+    DRPT_LAUNCH_CHECK();
+    const unsigned items = (unsigned)p.items;
+    if (p.qt == 64)
+      DRPT_TRY((u8 ? query_tile<uint8_t, 64>(a, items, s) : query_tile<float, 64>(a, items, s)));
+    else
+      DRPT_TRY((u8 ? query_tile<uint8_t, 16>(a, items, s) : query_tile<float, 16>(a, items, s)));
+  }
+  return launch_merge(a.ci, a.cd, a.nq, a.T, a.k, a.k, a.oi, a.od, s);
 }
 
 }  // namespace drpt

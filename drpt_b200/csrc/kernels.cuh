@@ -163,9 +163,37 @@ drpt_status launch_rerank(const void *X, int dtype, int d, const int32_t *visit,
 // ---- out-of-sample queries (k_query.cu) ---------------------------------------
 drpt_status launch_descend(const float *Pq, int64_t nq, int T, int gd, const float *medians,
                            int32_t *leaf, cudaStream_t s);
-drpt_status launch_query(const void *X, int dtype, int d, int64_t n, const void *Qx, int64_t nq,
-                         int T, const int32_t *order, const int32_t *goff, int nleaf,
-                         const int32_t *leaf, int k, int32_t *oi, float *od, cudaStream_t s);
+// How a block of queries runs, and the scratch it needs: `qt` queries per item
+// of the grouped form (0: the few-queries form, each leaf cut into `shares`),
+// `lists` sorted lists of k entries.
+struct QueryPlan {
+  int qt, shares;
+  int64_t lists, entries, buckets, items;
+};
+QueryPlan query_plan(int64_t nq, int T, int nleaf, int max_leaf, int k, bool aligned);
+
+struct QueryArgs {
+  const void *X;               // n x d indexed rows
+  int dtype;
+  int d;
+  int64_t n;
+  const void *Q;               // nq x d queries
+  int64_t nq;
+  int T;
+  const int32_t *order, *goff; // T x n, T x (nleaf + 1)
+  int nleaf;
+  const int32_t *leaf;         // nq x T
+  int k;
+  int32_t *ci;                 // plan.entries
+  float *cd;
+  // grouped form: pairs, buckets, buckets, plan.items, 1, pairs
+  int32_t *rank, *cnt, *off;
+  int4 *items;
+  int32_t *n_items, *list;
+  int32_t *oi;                 // nq x k
+  float *od;
+};
+drpt_status launch_query(const QueryArgs &a, const QueryPlan &p, cudaStream_t s);
 
 // ---- learned splits (k_learned.cu) ------------------------------------------
 constexpr int kLearnHidden = 64;
