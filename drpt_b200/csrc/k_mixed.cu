@@ -14,14 +14,14 @@
 //                       of the rounded row
 //   K9  k_tile_plan     row tiles of 128 points of every leaf
 //   K10 k_leaf_mma      per row tile: TMA-fed tcgen05 MMAs (BF16 x BF16 ->
-//                       FP32 in Tensor Memory, M = 128 rows, N = 64 columns
-//                       per tile, K = the padded dimension), epilogue scores
-//                       ||y||^2 - 2 x.y per column and keeps each row's KP
-//                       best in registers (threshold filter seeded from the
-//                       running list, per-thread shared-memory buffer,
-//                       bitonic sort + merge), then folds them into the
-//                       point's running list of the KP best distinct
-//                       candidates over the trees built so far
+//                       FP32 in Tensor Memory, M = 128 rows, N = 64 to 256
+//                       columns per tile, K = the padded dimension), epilogue
+//                       scores ||y||^2 - 2 x.y per column and keeps each
+//                       row's KP best in registers (threshold filter seeded
+//                       from the running list, per-thread shared-memory
+//                       buffer, sort + merge networks); k_fold_lists then
+//                       folds them into the point's running list of the KP
+//                       best distinct candidates over the trees built so far
 //   K11 k_rerank        per point: the running list's KP candidates rescored with the
 //                       exact sequential FP32 distance of the plain form, the
 //                       k best kept; candidates whose FP32 distance lies within
@@ -46,35 +46,46 @@ namespace {
 using namespace sm100;
 
 constexpr int kTM = 128;            // rows per tile (M)
-constexpr int kTN = 64;             // columns per tile (N) of the streamed form
-// Per list width KP and A layout: columns per tile (N), accumulator buffers
-// (together 128 TMEM columns), B-tile stages, per-row pending-key slots,
-// epilogue groups of four warps and the CTAs per SM the kernel is built for.
-// The epilogue bounds the kernel: with 16 keys per row and a resident A,
-// one group, 3 CTAs per SM (d <= 128: 68 KB of shared memory each) on one
-// 64-column B stage and 32 slots.  Measured slower on the 1M x 128 bench
-// build (leaf kernel, 6 trees): two groups taking the column tiles in turn
-// at 2 CTAs per SM (5.96 ms against 4.96: their split lists need more
-// flushes), three 32-column stages with four accumulators (5.35 ms: twice
-// the per-tile epilogue overhead), one group at 2 CTAs per SM with two or
-// three stages (5.48 ms).  With 32 keys or a streamed A: one group, 2 CTAs,
-// two stages, 64 or 32 slots.
-template <int KP, bool STREAM>
+// Four shapes of the leaf kernel, by how many 128-byte K blocks a row has.
+// In all of them the 128 rows of a tile (A) meet the leaf's columns in tiles
+// of `tn` (B) through a ring of stages of one K block each, into two
+// accumulators.
+//   0: kb <= 2, A resident, 64 columns, 3 CTAs per SM (32 keys per row: 2).
+//      The epilogue bounds it, so the warps per SM count.
+//   1: kb <= 4 and 16 keys, A resident (64 KB), 64 columns, 2 CTAs per SM.
+//   2: a stage holds a K block of A too, 128 columns, 2 CTAs per SM.
+//   3: kb >= kWideKb, as 2 with 256 columns, 1 CTA per SM.
+// Past shape 0 the feed from L2 bounds the kernel (64-column tiles with A
+// streamed took in 48 bytes per cycle and SM, of the 64 there are): per 64
+// columns and K block shape 1 fetches 8 KB, shape 2 16 KB, shape 3 12 KB,
+// where those tiles fetch 24.  An MMA of 64 columns also takes 48 cycles for
+// 32 cycles of work (it reads 6 KB of shared memory at 128 bytes per cycle);
+// of 128 or more it runs at its full rate.  Leaf kernels of the 60,000 x 784
+// u8 build (12 trees, 13 K blocks) 2.76 -> 1.37 ms, of 500,000 x 960 in E4M3
+// (32 trees, 8 K blocks) 49.9 -> 38 ms.  The line between 2 and 3: a build
+// with 8 K blocks takes 2.47 ms in shape 2 and 2.65 in shape 3, with 11 blocks
+// 2.52 and 2.54, with 15 blocks 4.32 and 4.11 (one CTA's four epilogue warps
+// are too few for short rows).  Measured slower: A resident on one CTA per SM
+// with 128 columns (8 blocks: 71.7 ms per E4M3 build against 65.6 streamed),
+// and A in Tensor Memory (such an MMA takes about 150 cycles at 64 columns).
+constexpr int kWideKb = 12;
+template <int KP, int SHAPE>
 struct MmaCfg {
-  static constexpr bool dense = KP == 16 && !STREAM;
-  static constexpr int tn = 64;
-  static constexpr int nacc = 128 / tn;
-  static constexpr int stages = dense ? 1 : 2;
-  static constexpr int slots = KP == 16 ? 32 : 64;
-  static constexpr int groups = 1;
-  static constexpr int epi_warps = 4 * groups;
+  static constexpr int tn = SHAPE <= 1 ? 64 : (SHAPE == 2 ? 128 : 256);
+  static constexpr bool stream = SHAPE >= 2;
+  static constexpr int slots = KP == 16 ? 32 : 64;  // pending-key slots per row
+  static constexpr int vw = SHAPE <= 2 ? 32 : 64;   // columns read from TMEM at a time
+  static constexpr uint32_t stage = (stream ? kTM * 128 : 0) + tn * 128;  // bytes
+  static constexpr int epi_warps = 4;
   static constexpr int threads = 32 * (epi_warps + 2);
-  static constexpr int min_blocks = dense ? 3 : 2;
+  static constexpr int min_blocks = SHAPE == 0 ? (KP == 16 ? 3 : 2) : (SHAPE <= 2 ? 2 : 1);
 };
+constexpr int kMaxStages = 8;
 constexpr int kColBits = 13;        // low key bits holding the column in the leaf
 constexpr uint32_t kColMask = (1u << kColBits) - 1;
 constexpr int kMaxLeaf = 1 << kColBits;  // largest leaf the key can address
 constexpr int kCheck = 16;          // columns between flush checks
+
 constexpr int kCentreRows = 64;     // rows averaged for a leaf's centre
 
 __device__ __forceinline__ bool before(float da, int32_t ia, float db, int32_t ib) {
@@ -487,20 +498,19 @@ __device__ __forceinline__ void key_cmp_swap(float *d, int a, int b) {  // d[a] 
   d[b] = y;
 }
 
+// Batcher's odd-even merge sort (K. E. Batcher, "Sorting networks and their
+// applications", 1968), ascending: 63 exchanges for 16 keys where the bitonic
+// network takes 80 (19 against 24 for 8).
 template <int N>
 __device__ __forceinline__ void key_sort(float *d) {
 #pragma unroll
-  for (int k = 2; k <= N; k <<= 1)
+  for (int p = 1; p < N; p <<= 1)
 #pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1)
+    for (int k = p; k > 0; k >>= 1)
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-        const int l = i ^ j;
-        if (l > i) {
-          if ((i & k) == 0) key_cmp_swap(d, i, l);
-          else key_cmp_swap(d, l, i);
-        }
-      }
+      for (int i = 0; i + k < N; ++i)
+        if (i >= k % p && (i - k % p) % (2 * k) < k && i / (2 * p) == (i + k) / (2 * p))
+          key_cmp_swap(d, i, i + k);
 }
 
 // L (ascending, N) <- the N smallest of L and S (ascending, M <= N).
@@ -534,43 +544,38 @@ __device__ __forceinline__ void key_insert(float *L, float key) {
 
 // Shared-memory layout.  Every operand tile is rows of 128 bytes (64 BF16 or
 // 128 E4M3 values of one 128-byte K block), 128-byte swizzled, 1024-byte
-// aligned.
-//   resident A (kb <= 2): A = kb K blocks of the 128 rows, loaded once per row
-//     tile; `stages` stages of the kb K blocks of a tn-column B tile;
-//   streamed A (larger kb): kSStages stages, each one K block of A (16 KB)
-//     and of B (8 KB), so A is re-read from L2 for every column tile.
-constexpr int kSStages = 3;
-constexpr uint32_t kStreamA = kTM * 128, kStreamStage = kTM * 128 + kTN * 128;
-
+// aligned: resident A (kb K blocks of 16 KB), then the ring of stages.
 struct MmaSmem {
-  uint32_t a_off, b_off, buf_off, nrm_off, scl_off, thr_off, bar_off, total;
+  uint32_t b_off, buf_off, nrm_off, scl_off, bar_off, total;
+  int stages;
 };
 
-__host__ __device__ inline MmaSmem mma_smem_layout(int kb, bool stream, int stages, int slots,
-                                                   int tn, int groups) {
+template <int KP, int SHAPE>
+__host__ __device__ inline MmaSmem mma_smem_layout(int kb, bool fp8) {
+  using Cfg = MmaCfg<KP, SHAPE>;
+  constexpr uint32_t rest = kTM * Cfg::slots * 4 + 2 * 4 * Cfg::tn * 4 + (2 * kMaxStages + 5) * 8 + 16;
+  // a third (half, all) of the SM's 228 KB, less 1 KB per CTA for the system
+  // and 1 KB to align the tiles
+  constexpr uint32_t room = 228 * 1024 / Cfg::min_blocks - 2048;
   MmaSmem L;
-  L.a_off = 0;
-  if (stream) {
-    L.b_off = kStreamA;  // inside each stage
-    L.buf_off = kSStages * kStreamStage;
-  } else {
-    L.b_off = L.a_off + (uint32_t)kb * kTM * 128;
-    L.buf_off = L.b_off + (uint32_t)stages * kb * tn * 128;
-  }
-  L.nrm_off = L.buf_off + kTM * (uint32_t)slots * groups * 4;
-  L.scl_off = L.nrm_off + 4 * groups * (uint32_t)tn * 4;
-  L.thr_off = L.scl_off + 4 * groups * (uint32_t)tn * 4;
-  L.bar_off = L.thr_off + (uint32_t)groups * kTM * 4;
-  L.total = L.bar_off + 24 * 8 + 16;
+  L.b_off = Cfg::stream ? 0 : (uint32_t)kb * kTM * 128;
+  const uint32_t fixed = L.b_off + rest - (fp8 ? 0 : 4 * Cfg::tn * 4);
+  const int fit = fixed < room ? (int)((room - fixed) / Cfg::stage) : 0;
+  L.stages = fit < kMaxStages ? fit : kMaxStages;
+  L.buf_off = L.b_off + L.stages * Cfg::stage;
+  L.nrm_off = L.buf_off + kTM * (uint32_t)Cfg::slots * 4;
+  L.scl_off = L.nrm_off + 4 * Cfg::tn * 4;
+  L.bar_off = L.scl_off + (fp8 ? 4 * Cfg::tn * 4 : 0);
+  L.total = L.bar_off + (2 * kMaxStages + 5) * 8 + 16;
   return L;
 }
 
-// KP: candidates kept per row and tree.  STREAM: streamed A.  FP8: E4M3
-// operands with per-row scales `scl` (scores are then scaled by the row's and
-// the column's scale); otherwise BF16.
-template <int KP, bool STREAM, bool FP8>
-__global__ void __launch_bounds__(MmaCfg<KP, STREAM>::threads,
-                                  MmaCfg<KP, STREAM>::min_blocks) k_leaf_mma(
+// KP: candidates kept per row and tree.  FP8: E4M3 operands with per-row
+// scales `scl` (scores are then scaled by the row's and the column's scale);
+// otherwise BF16.
+template <int KP, int SHAPE, bool FP8>
+__global__ void __launch_bounds__(MmaCfg<KP, SHAPE>::threads,
+                                  MmaCfg<KP, SHAPE>::min_blocks) k_leaf_mma(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     const int32_t *__restrict__ goff, const int32_t *__restrict__ order,
     const float *__restrict__ nrm, const float *__restrict__ scl,
@@ -581,29 +586,26 @@ __global__ void __launch_bounds__(MmaCfg<KP, STREAM>::threads,
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t *smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
-  using Cfg = MmaCfg<KP, STREAM>;
-  constexpr int kBufSlots = Cfg::slots;
-  constexpr int TN = Cfg::tn, NACC = Cfg::nacc, G = Cfg::groups, EPI = Cfg::epi_warps;
-  static_assert(!STREAM || TN == kTN, "streamed stages hold kTN-column B blocks");
-  static_assert(NACC % G == 0, "a group owns whole accumulators");
-  const MmaSmem L = mma_smem_layout(kb, STREAM, Cfg::stages, Cfg::slots, TN, G);
-  uint8_t *sA = smem + L.a_off;
+  using Cfg = MmaCfg<KP, SHAPE>;
+  constexpr int kBufSlots = Cfg::slots, EPI = Cfg::epi_warps, TN = Cfg::tn;
+  constexpr bool STREAM = Cfg::stream;
+  const MmaSmem L = mma_smem_layout<KP, SHAPE>(kb, FP8);
+  const int NS = L.stages;
+  uint8_t *sA = smem;
   uint8_t *sB = smem + L.b_off;
-  uint32_t *buf = reinterpret_cast<uint32_t *>(smem + L.buf_off);  // [group][slot][row] keys
-  float *thr_sh = reinterpret_cast<float *>(smem + L.thr_off);  // [group][row] KP-th best key
+  uint32_t *buf = reinterpret_cast<uint32_t *>(smem + L.buf_off);  // [slot][row] keys
   float *nbuf = reinterpret_cast<float *>(smem + L.nrm_off);  // [warp][TN] column norms of a tile
   float *sbuf = reinterpret_cast<float *>(smem + L.scl_off);  // [warp][TN] column scales (FP8)
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bar_off);
-  static_assert(kSStages <= 4 && Cfg::stages <= 4 && NACC <= 4, "barrier slots");
   uint64_t *full_a = bars + 0;
-  uint64_t *full_b = bars + 1;     // up to 4 stages
-  uint64_t *empty_b = bars + 5;    // up to 4 stages
-  uint64_t *acc_full = bars + 9;   // up to 4 accumulators
-  uint64_t *acc_empty = bars + 13; // up to 4 accumulators
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 24);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 24) + 1;
-  constexpr int NS = STREAM ? kSStages : Cfg::stages;
+  uint64_t *acc_full = bars + 1;   // 2 accumulators
+  uint64_t *acc_empty = bars + 3;  // 2 accumulators
+  uint64_t *full_b = bars + 5;     // NS stages
+  uint64_t *empty_b = full_b + kMaxStages;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(empty_b + kMaxStages);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   constexpr int kKE = FP8 ? 128 : 64;  // elements per 128-byte K block
+  constexpr uint32_t kStageA = STREAM ? kTM * 128 : 0;
 
   const int u = blockIdx.x;
   if (u >= *n_tiles) return;  // uniform for the whole block
@@ -615,7 +617,6 @@ __global__ void __launch_bounds__(MmaCfg<KP, STREAM>::threads,
     return;  // uniform for the whole block
   }
   const int nct = (m + TN - 1) / TN;
-  const uint32_t a_bytes = (uint32_t)kb * kTM * 128, b_bytes = (uint32_t)kb * TN * 128;
 
   if (threadIdx.x == 0) {
     mbar_init(full_a, 1);
@@ -623,15 +624,14 @@ __global__ void __launch_bounds__(MmaCfg<KP, STREAM>::threads,
       mbar_init(full_b + s, 1);
       mbar_init(empty_b + s, 1);
     }
-    for (int b = 0; b < NACC; ++b) {
+    for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full + b, 1);
-      mbar_init(acc_empty + b, 4 * 32);  // the owning group's 128 threads
+      mbar_init(acc_empty + b, EPI * 32);
     }
     *abort_flag = 0;
     fence_barrier_init();
   }
-  for (int i = threadIdx.x; i < G * kTM; i += blockDim.x) thr_sh[i] = __int_as_float(0x7f800000);
-  if (warp == EPI + 1) tmem_alloc(tmem_slot, 128);  // NACC accumulators x TN columns
+  if (warp == EPI + 1) tmem_alloc(tmem_slot, 2 * TN);
   if (warp == EPI && lane == 0) {
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmB);
@@ -642,36 +642,31 @@ __global__ void __launch_bounds__(MmaCfg<KP, STREAM>::threads,
   const uint32_t tmem = *tmem_slot;
 
   if (warp == EPI) {
-    // ---- TMA producer
+    // ---- TMA producer: stage i = (column tile c, K block q), i = c * kb + q
     if (lane == 0) {
-      if constexpr (STREAM) {
-        // stage i = (column tile c, K block q) with i = c * kb + q
-        const int total = nct * kb;
-        for (int i = 0; i < total && !*abort_flag; ++i) {
-          const int s = i % NS, c = i / kb, q = i - c * kb;
-          if (i >= NS && !mbar_wait(empty_b + s, ((i / NS) - 1) & 1)) {
-            *abort_flag = 1;
-            break;
-          }
-          uint8_t *st = smem + (size_t)s * kStreamStage;
-          mbar_arrive_expect_tx(full_b + s, kStreamStage);
-          tma_load_2d(st, &tmA, full_b + s, q * kKE, lo + r0);
-          tma_load_2d(st + kStreamA, &tmB, full_b + s, q * kKE, lo + c * TN);
-        }
-      } else {
-        mbar_arrive_expect_tx(full_a, a_bytes);
+      if constexpr (!STREAM) {
+        mbar_arrive_expect_tx(full_a, (uint32_t)kb * kTM * 128);
         for (int q = 0; q < kb; ++q)
           tma_load_2d(sA + q * kTM * 128, &tmA, full_a, q * kKE, lo + r0);
-        for (int c = 0; c < nct && !*abort_flag; ++c) {
-          const int s = c % NS;
-          if (c >= NS && !mbar_wait(empty_b + s, ((c / NS) - 1) & 1)) {
-            *abort_flag = 1;
-            break;
-          }
-          uint8_t *dst = sB + s * b_bytes;
-          mbar_arrive_expect_tx(full_b + s, b_bytes);
-          for (int q = 0; q < kb; ++q)
-            tma_load_2d(dst + q * TN * 128, &tmB, full_b + s, q * kKE, lo + c * TN);
+      }
+      const int total = nct * kb;
+      int s = 0, ph = 1, q = 0, y = lo;
+      for (int i = 0; i < total && !*abort_flag; ++i) {
+        if (i >= NS && !mbar_wait(empty_b + s, ph)) {
+          *abort_flag = 1;
+          break;
+        }
+        uint8_t *st = sB + s * Cfg::stage;
+        mbar_arrive_expect_tx(full_b + s, Cfg::stage);
+        if constexpr (STREAM) tma_load_2d(st, &tmA, full_b + s, q * kKE, lo + r0);
+        tma_load_2d(st + kStageA, &tmB, full_b + s, q * kKE, y);
+        if (++s == NS) {
+          s = 0;
+          ph ^= 1;
+        }
+        if (++q == kb) {
+          q = 0;
+          y += TN;
         }
       }
     }
@@ -680,47 +675,33 @@ __global__ void __launch_bounds__(MmaCfg<KP, STREAM>::threads,
     // 32 E4M3 values, 32 bytes each)
     if (lane == 0) {
       constexpr uint32_t idesc = FP8 ? idesc_e4m3_f32(kTM, TN) : idesc_bf16_f32(kTM, TN);
-      auto mma = [&](uint32_t d, uint64_t ad, uint64_t bd, uint32_t acc) {
-        if constexpr (FP8) mma_e4m3(d, ad, bd, idesc, acc);
-        else mma_bf16(d, ad, bd, idesc, acc);
-      };
-      bool ok = true;
-      if constexpr (STREAM) {
-        for (int c = 0; ok && c < nct && !*abort_flag; ++c) {
-          const int b = c % NACC;
-          if (c >= NACC) ok = mbar_wait(acc_empty + b, ((c / NACC) - 1) & 1);
-          for (int q = 0; ok && q < kb; ++q) {
-            const int i = c * kb + q, s = i % NS;
-            ok = mbar_wait(full_b + s, (i / NS) & 1);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t as = smem_u32(smem + (size_t)s * kStreamStage), bs = as + kStreamA;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              mma(tmem + b * TN, desc_k_sw128(as + k * 32), desc_k_sw128(bs + k * 32),
-                  (q | k) ? 1u : 0u);
-            mma_commit(empty_b + s);
-          }
-          if (ok) mma_commit(acc_full + b);
-        }
-      } else {
-        const uint32_t a_base = smem_u32(sA), b_base = smem_u32(sB);
-        ok = mbar_wait(full_a, 0);
-        for (int c = 0; ok && c < nct && !*abort_flag; ++c) {
-          const int s = c % NS, b = c % NACC;
-          ok = mbar_wait(full_b + s, (c / NS) & 1);
-          if (ok && c >= NACC) ok = mbar_wait(acc_empty + b, ((c / NACC) - 1) & 1);
+      const uint32_t a_base = smem_u32(sA), b_base = smem_u32(sB);
+      bool ok = STREAM || mbar_wait(full_a, 0);
+      int s = 0, ph = 0;
+      for (int c = 0; ok && c < nct && !*abort_flag; ++c) {
+        const int b = c & 1;
+        if (c > 1) ok = mbar_wait(acc_empty + b, ((c >> 1) - 1) & 1);
+        for (int q = 0; ok && q < kb; ++q) {
+          ok = mbar_wait(full_b + s, ph);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t bs = b_base + s * b_bytes;
-          for (int q = 0; q < kb; ++q)
+          const uint32_t st = b_base + s * Cfg::stage;
+          const uint64_t ad = desc_k_sw128(STREAM ? st : a_base + q * kTM * 128);
+          const uint64_t bd = desc_k_sw128(st + kStageA);
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              mma(tmem + b * TN, desc_k_sw128(a_base + q * kTM * 128 + k * 32),
-                  desc_k_sw128(bs + q * TN * 128 + k * 32), (q | k) ? 1u : 0u);
+          for (int k = 0; k < 4; ++k) {  // 32 bytes further: 2 in the descriptors' address
+            if constexpr (FP8)
+              mma_e4m3(tmem + b * TN, ad + 2 * k, bd + 2 * k, idesc, (q | k) ? 1u : 0u);
+            else
+              mma_bf16(tmem + b * TN, ad + 2 * k, bd + 2 * k, idesc, (q | k) ? 1u : 0u);
+          }
           mma_commit(empty_b + s);
-          mma_commit(acc_full + b);
+          if (++s == NS) {
+            s = 0;
+            ph ^= 1;
+          }
         }
+        if (ok) mma_commit(acc_full + b);
       }
       if (!ok) *abort_flag = 1;
     }
@@ -732,15 +713,10 @@ __global__ void __launch_bounds__(MmaCfg<KP, STREAM>::threads,
     // row's current KP-th best go to a slot-major shared buffer
     // (conflict-free: consecutive rows are consecutive words); when any row
     // of the warp has too many pending, every row sorts its pending keys in
-    // batches of 16 and merges them into its sorted list of KP keys with a
-    // bitonic network.  With two groups, group g takes the column tiles
-    // c = g, g + 2, ... (accumulator g) and keeps its own list per row; each
-    // group filters with the smaller of the groups' KP-th best keys (a key
-    // above another group's KP-th best cannot be among the KP best of the
-    // union), and group 0 merges the lists at the end.
-    const int grp = warp / 4, wq = warp % 4;
-    const int row = wq * 32 + lane;
+    // batches and merges them into its sorted list of KP keys.
+    const int row = warp * 32 + lane;
     const bool rvalid = r0 + row < m;
+    const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
     float td[KP];
 #pragma unroll
     for (int j = 0; j < KP; ++j) td[j] = __int_as_float(0x7f800000);
@@ -758,13 +734,12 @@ __global__ void __launch_bounds__(MmaCfg<KP, STREAM>::threads,
       if (tree > 0) thr = run_dist[(int64_t)my_pt * KP + KP - 1] - nr;
     }
     const float thr0 = thr;
-    const uint32_t my_col = (uint32_t)(r0 + row);  // the row's own point, dropped when read
     // Pending keys: a passing key is stored at the next free slot of one of
     // two per-row lanes of the buffer (even and odd columns, two independent
     // append chains) by a predicated shared-memory store, no branch; slot
     // addresses are 32-bit shared-window offsets.
     constexpr int kChains = 2, kLane = kBufSlots / kChains, kPerBatch = 16 / kChains;
-    uint32_t *const pbase = buf + grp * kBufSlots * kTM + row;
+    uint32_t *const pbase = buf + row;
     const uint32_t abase = smem_u32(pbase);
     uint32_t aslot[kChains], alim[kChains];
 #pragma unroll
@@ -775,113 +750,129 @@ __global__ void __launch_bounds__(MmaCfg<KP, STREAM>::threads,
       // stay inside its kLane slots
       alim[q] = aslot[q] + (kLane - kCheck / kChains) * kTM * 4;
     }
-    auto pending = [&](int q) {
-      return (int)((aslot[q] - abase - q * kLane * kTM * 4) / (kTM * 4));
-    };
-    auto flush = [&]() {
-      int cnt[kChains], mine = 0;
+    // The flush is a few hundred instructions of unrolled networks.  The scan
+    // below is written so that the kernel holds one copy of it: with a copy at
+    // every check (nine) the warps waited for instructions.  With the shorter
+    // networks, the one-instruction key and the predicated append: 121.5 M ->
+    // 99 M warp instructions per tree at 262,144 x 128, 213 -> 185 us under
+    // the profiler; the 1M x 128 build of 6 trees 7.20 -> 6.76 ms.
+    const int own = r0 + warp * 32;  // columns own .. own + 31: the warp's own points
+    int seen = 0;                    // columns below it are flushed
+    auto flush = [&](int upto) {
+      int cnt[kChains], mx = 0;
 #pragma unroll
       for (int q = 0; q < kChains; ++q) {
-        cnt[q] = pending(q);
-        mine = max(mine, cnt[q]);
+        cnt[q] = (int)((aslot[q] - abase) / (kTM * 4)) - q * kLane;
+        mx = max(mx, cnt[q]);
       }
-      const int mx = __reduce_max_sync(kFull, mine);
-      if (mx <= 3) {
-        // few pending keys (the common case once a threshold is set): insert
-        // them one by one (2 KP min/max each) rather than sort a batch of 16
-        // and merge it (about 240); the kept keys are the same
+      mx = __reduce_max_sync(kFull, mx);
+      if (own < upto && own + 32 > seen) {
+        // the row's own point may be pending (in one of the row's tiles):
+        // its key becomes infinite (eight slots read at a time; those past
+        // the pending ones are not changed)
+#pragma unroll 1
+        for (int e0 = 0; e0 < mx; e0 += 4) {
+          uint32_t key[4][kChains];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int q = 0; q < kChains; ++q) key[e][q] = pbase[(q * kLane + e0 + e) * kTM];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int q = 0; q < kChains; ++q)
+              if (e0 + e < cnt[q] && (key[e][q] & kColMask) == (uint32_t)(own + lane))
+                pbase[(q * kLane + e0 + e) * kTM] = 0x7f800000u;
+        }
+      }
+      seen = upto;
+      // W keys of each chain from slot `base` on (+inf past its pending
+      // ones), sorted and merged into the list
+      auto take = [&](int base, auto width) {
+        constexpr int W = decltype(width)::value;
+        float sd[kChains * W];
 #pragma unroll
         for (int q = 0; q < kChains; ++q)
-          for (int slot = 0; slot < mx; ++slot) {
-            uint32_t key = 0x7f800000u;
-            if (slot < cnt[q]) key = pbase[(q * kLane + slot) * kTM];
-            if ((key & kColMask) == my_col && key != 0x7f800000u) key = 0x7f800000u;
-            key_insert<KP>(td, __uint_as_float(key));
-          }
-      }
-      for (int base = 0; mx > 3 && base < mx; base += kPerBatch) {
-        float sd[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const int q = e / kPerBatch, slot = base + e % kPerBatch;
-          uint32_t key = 0x7f800000u;
-          if (slot < cnt[q]) key = pbase[(q * kLane + slot) * kTM];
-          if ((key & kColMask) == my_col && key != 0x7f800000u) key = 0x7f800000u;
-          sd[e] = __uint_as_float(key);
+          for (int e = 0; e < W; ++e) {
+            sd[q * W + e] = __int_as_float(0x7f800000);
+            if (base + e < cnt[q])
+              sd[q * W + e] = __uint_as_float(pbase[(q * kLane + base + e) * kTM]);
+          }
+        key_sort<kChains * W>(sd);
+        key_merge_into<KP, kChains * W>(td, sd);
+      };
+      int base = 0;
+      constexpr int kTail = KP == 16 ? 3 : 2;
+#pragma unroll 1
+      for (; mx - base > kTail; base += kPerBatch)
+        take(base, std::integral_constant<int, kPerBatch>{});
+      // a rest of a few keys a chain one by one (2 KP min/max each): cheaper
+      // than a batch of 16 and its merge (about 200); the kept keys are the same
+#pragma unroll 1
+      for (; base < mx; ++base)
+#pragma unroll
+        for (int q = 0; q < kChains; ++q) {
+          float key = __int_as_float(0x7f800000);
+          if (base < cnt[q]) key = __uint_as_float(pbase[(q * kLane + base) * kTM]);
+          key_insert<KP>(td, key);
         }
-        key_sort<16>(sd);
-        key_merge_into<KP, 16>(td, sd);
-      }
 #pragma unroll
       for (int q = 0; q < kChains; ++q) aslot[q] = abase + q * kLane * kTM * 4;
-      float lim = td[KP - 1];
-      if constexpr (G > 1) {
-        volatile float *ts = thr_sh;
-        ts[grp * kTM + row] = lim;
-#pragma unroll
-        for (int g2 = 0; g2 < G; ++g2)
-          if (g2 != grp) lim = fminf(lim, ts[g2 * kTM + row]);
-      }
-      thr = fminf(thr0, lim);
+      thr = fminf(thr0, td[KP - 1]);
     };
     // key = the score's high bits and the column bits of the packed norm
     // (one bit-select), stored only when the score beats the threshold
     auto append = [&](uint32_t &slot, float sv, float ncp) {
-      const uint32_t key = (__float_as_uint(sv) & ~kColMask) | (__float_as_uint(ncp) & kColMask);
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t"
-          "setp.lt.f32 p, %1, %2;\n\t"
-          "@p st.shared.u32 [%0], %3;\n\t"
-          "@p add.u32 %0, %0, %4;\n\t}"
-          : "+r"(slot)
-          : "f"(sv), "f"(thr), "r"(key), "n"(kTM * 4)
-          : "memory");
-    };
-    // one 32-column chunk of scores; the packed norms (and E4M3 scales) of
-    // each kCheck columns are read into registers before that group's
-    // stores, so the loads do not wait behind them
-    auto scan = [&](const float *v, const float *wn, const float *ws) {
-#pragma unroll
-      for (int h = 0; h < 32; h += kCheck) {
-        float nc[kCheck], sc[kCheck];
-#pragma unroll
-        for (int j4 = 0; j4 < kCheck; j4 += 4) {
-          const float4 a = *reinterpret_cast<const float4 *>(wn + h + j4);
-          nc[j4] = a.x;
-          nc[j4 + 1] = a.y;
-          nc[j4 + 2] = a.z;
-          nc[j4 + 3] = a.w;
-          if constexpr (FP8) {
-            const float4 b = *reinterpret_cast<const float4 *>(ws + h + j4);
-            sc[j4] = b.x;
-            sc[j4 + 1] = b.y;
-            sc[j4 + 2] = b.z;
-            sc[j4 + 3] = b.w;
-          }
-        }
-        (void)sc;
-#pragma unroll
-        for (int e = 0; e < kCheck; e += 2) {
-          const int j = h + e;
-          float2 sv;
-          if constexpr (FP8) {
-            sv.x = fmaf(m2s * sc[e], v[j], nc[e]);
-            sv.y = fmaf(m2s * sc[e + 1], v[j + 1], nc[e + 1]);
-          } else {
-            // two scores per packed FP32x2 multiply-add
-            sv = fma2(make_float2(v[j], v[j + 1]), make_float2(-2.0f, -2.0f),
-                      make_float2(nc[e], nc[e + 1]));
-          }
-          append(aslot[j % kChains], sv.x, nc[e]);
-          append(aslot[(j + 1) % kChains], sv.y, nc[e + 1]);
-        }
-        bool over = false;
-#pragma unroll
-        for (int q = 0; q < kChains; ++q) over |= aslot[q] > alim[q];
-        if (__any_sync(kFull, over)) flush();
+      uint32_t key;  // one bit-select (0xD8: sv where the mask is 0, else ncp)
+      asm("lop3.b32 %0, %1, %2, %3, 0xD8;"
+          : "=r"(key)
+          : "r"(__float_as_uint(sv)), "r"(__float_as_uint(ncp)), "r"(kColMask));
+      if (sv < thr) {  // becomes two predicated instructions
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(slot), "r"(key) : "memory");
+        slot += kTM * 4;
       }
     };
-    const uint32_t lane_base = tmem + ((uint32_t)(wq * 32) << 16);
+    // kCheck columns of scores; their packed norms (and E4M3 scales) are read
+    // into registers before the stores, so the loads do not wait behind them.
+    // Returns whether a chain is too full for another kCheck columns.
+    auto scan = [&](const float *v, const float *wn, const float *ws) {
+      float nc[kCheck], sc[kCheck];
+#pragma unroll
+      for (int j4 = 0; j4 < kCheck; j4 += 4) {
+        const float4 a = *reinterpret_cast<const float4 *>(wn + j4);
+        nc[j4] = a.x;
+        nc[j4 + 1] = a.y;
+        nc[j4 + 2] = a.z;
+        nc[j4 + 3] = a.w;
+        if constexpr (FP8) {
+          const float4 b = *reinterpret_cast<const float4 *>(ws + j4);
+          sc[j4] = b.x;
+          sc[j4 + 1] = b.y;
+          sc[j4 + 2] = b.z;
+          sc[j4 + 3] = b.w;
+        }
+      }
+      (void)sc;
+#pragma unroll
+      for (int e = 0; e < kCheck; e += 2) {
+        float2 sv;
+        if constexpr (FP8) {
+          sv.x = fmaf(m2s * sc[e], v[e], nc[e]);
+          sv.y = fmaf(m2s * sc[e + 1], v[e + 1], nc[e + 1]);
+        } else {
+          // two scores per packed FP32x2 multiply-add
+          sv = fma2(make_float2(v[e], v[e + 1]), make_float2(-2.0f, -2.0f),
+                    make_float2(nc[e], nc[e + 1]));
+        }
+        append(aslot[e % kChains], sv.x, nc[e]);
+        append(aslot[(e + 1) % kChains], sv.y, nc[e + 1]);
+      }
+      bool over = false;
+#pragma unroll
+      for (int q = 0; q < kChains; ++q) over |= aslot[q] > alim[q];
+      return over;
+    };
     // column norms (and E4M3 scales) of a tile: lane l holds columns l and
     // l + 32, loaded one tile ahead; columns past the leaf carry an infinite
     // norm (a NaN once packed) and so never pass
@@ -896,12 +887,13 @@ __global__ void __launch_bounds__(MmaCfg<KP, STREAM>::threads,
         if constexpr (FP8) ps[h] = in ? __ldg(scl + lo + col) : 0.0f;
       }
     };
-    load_cols(grp);
-    for (int c = grp; c < nct; c += G) {
-      const int b = c % NACC;
+    load_cols(0);
+    float *wn = nbuf + warp * TN;
+    float *ws = sbuf + warp * TN;
+#pragma unroll 1
+    for (int c = 0; c < nct; ++c) {
+      const int b = c & 1;
       // this tile's column norms, staged per warp (16-byte aligned reads)
-      float *wn = nbuf + warp * TN;
-      float *ws = sbuf + warp * TN;
       __syncwarp();
 #pragma unroll
       for (int h = 0; h < TN / 32; ++h) {
@@ -914,40 +906,65 @@ __global__ void __launch_bounds__(MmaCfg<KP, STREAM>::threads,
         if constexpr (FP8) ws[h * 32 + lane] = ps[h];
       }
       __syncwarp();
-      load_cols(c + G);
-      if (!__all_sync(kFull, mbar_wait(acc_full + b, (c / NACC) & 1))) {
+      load_cols(c + 1);
+      if (!__all_sync(kFull, mbar_wait(acc_full + b, (c >> 1) & 1))) {
         *abort_flag = 1;
         break;
       }
       tc_fence_after();
+      constexpr int VW = Cfg::vw;
+#pragma unroll 1
+      for (int q = 0; q < TN; q += VW) {
+        float v[VW];
 #pragma unroll
-      for (int q = 0; q < TN / 32; ++q) {
-        float v[32];
-        tmem_ld32(lane_base + b * TN + q * 32, v);
-        scan(v, wn + q * 32, ws + q * 32);
-      }
-      tc_fence_before();
-      mbar_arrive(acc_empty + b);
-    }
-    flush();
-    if constexpr (G > 1) {
-      // groups g > 0 hand their sorted lists to group 0 through their own
-      // buffer slots (KP <= slots); a barrier over the epilogue warps only
-      if (grp > 0) {
-#pragma unroll
-        for (int j = 0; j < KP; ++j) pbase[j * kTM] = __float_as_uint(td[j]);
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(EPI * 32) : "memory");
-      if (grp == 0) {
-        for (int g2 = 1; g2 < G; ++g2) {
-          float sd[KP];
-#pragma unroll
-          for (int j = 0; j < KP; ++j) sd[j] = __uint_as_float(buf[(g2 * kBufSlots + j) * kTM + row]);
-          key_merge_into<KP, KP>(td, sd);
+        for (int i = 0; i < VW; i += 32) tmem_ld32(lane_base + b * TN + q + i, v + i);
+        if (q + VW == TN) {  // the accumulator is in registers: the next tile may have it
+          tc_fence_before();
+          mbar_arrive(acc_empty + b);
+        }
+        // groups of kCheck columns, one after the other; a group that leaves a
+        // chain too full goes to the one flush and on with the next group
+        auto group = [&](int g) {
+          return __any_sync(kFull, scan(v + g * kCheck, wn + q + g * kCheck,
+                                        ws + q + g * kCheck)) != 0;
+        };
+        const int done = c * TN + q;
+        if constexpr (VW == 32) {
+          bool last = false;
+          if (!group(0)) goto second;
+        full:
+          flush(done + (last ? 32 : kCheck));
+          if (last) continue;
+        second:
+          last = true;
+          if (group(1) || done + 32 == nct * TN) goto full;
+        } else {
+          int h = 0;
+        next:
+          bool over = false;
+          switch (h) {
+            case 0:
+              h = kCheck;
+              if ((over = group(0))) break;
+              [[fallthrough]];
+            case kCheck:
+              h = 2 * kCheck;
+              if ((over = group(1))) break;
+              [[fallthrough]];
+            case 2 * kCheck:
+              h = 3 * kCheck;
+              if ((over = group(2))) break;
+              [[fallthrough]];
+            default:
+              h = 4 * kCheck;
+              over = group(3);
+          }
+          if (over || done + h == nct * TN) flush(done + h);
+          if (h < VW) goto next;
         }
       }
     }
-    if (grp == 0 && rvalid) {
+    if (rvalid) {
       // this tree's list, keys back to (squared distance, point id), already
       // ascending by key, i.e. by distance: tree 0's is the running list;
       // later trees' go to the tree list, which k_fold_lists merges into the
@@ -978,7 +995,7 @@ __global__ void __launch_bounds__(MmaCfg<KP, STREAM>::threads,
   __syncthreads();
   if (warp == EPI + 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, 128);
+    tmem_dealloc(tmem, 2 * TN);
   }
   if (threadIdx.x == 0 && *abort_flag) atomicOr(err, 1);
 }
@@ -1296,21 +1313,21 @@ void stage_d(const LeafStageArgs &a, bool means, cudaStream_t s) {
   else stage_t<T, 8>(a, means, s);
 }
 
-template <int KP, bool STREAM, bool FP8>
+template <int KP, int SHAPE, bool FP8>
 drpt_status mma_t(const MixedTreeArgs &a, const CUtensorMap &tmA, int kb, cudaStream_t s) {
-  using Cfg = MmaCfg<KP, STREAM>;
+  using Cfg = MmaCfg<KP, SHAPE>;
   CUtensorMap tmB;
   DRPT_TRY(make_tmap(&tmB, a.Xb, a.n, a.d_pad, Cfg::tn, a.fp8));
-  const MmaSmem L = mma_smem_layout(kb, STREAM, Cfg::stages, Cfg::slots, Cfg::tn, Cfg::groups);
+  const MmaSmem L = mma_smem_layout<KP, SHAPE>(kb, FP8);
   const size_t smem = L.total + 1024;
-  if (smem > 227 * 1024) {
-    set_error("mixed leaf kernel: %zu bytes of shared memory needed", smem);
+  if (L.stages < 1) {
+    set_error("mixed leaf kernel: no room for %d K blocks", kb);
     return DRPT_ERR_UNSUPPORTED;
   }
   const unsigned grid = (unsigned)(ceil_div(a.n, kTM) + a.nleaf);
-  DRPT_CUDA(cudaFuncSetAttribute(k_leaf_mma<KP, STREAM, FP8>,
+  DRPT_CUDA(cudaFuncSetAttribute(k_leaf_mma<KP, SHAPE, FP8>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_leaf_mma<KP, STREAM, FP8><<<grid, Cfg::threads, smem, s>>>(
+  k_leaf_mma<KP, SHAPE, FP8><<<grid, Cfg::threads, smem, s>>>(
       tmA, tmB, a.goff, a.order, a.nrm, a.scl, a.tile_leaf, a.tile_r0, a.n_tiles, kb, a.tree,
       a.cand_idx, a.cand_dist, a.tree_idx, a.tree_dist, a.err);
   DRPT_LAUNCH_CHECK();
@@ -1318,14 +1335,18 @@ drpt_status mma_t(const MixedTreeArgs &a, const CUtensorMap &tmA, int kb, cudaSt
   return DRPT_OK;
 }
 
+template <int KP, bool FP8>
+drpt_status mma_shaped(const MixedTreeArgs &a, const CUtensorMap &tmA, int kb, cudaStream_t s) {
+  if (kb <= 2) return mma_t<KP, 0, FP8>(a, tmA, kb, s);
+  if constexpr (KP == 16)
+    if (kb <= 4) return mma_t<KP, 1, FP8>(a, tmA, kb, s);
+  if (kb < kWideKb) return mma_t<KP, 2, FP8>(a, tmA, kb, s);
+  return mma_t<KP, 3, FP8>(a, tmA, kb, s);
+}
+
 template <int KP>
 drpt_status mma_kp(const MixedTreeArgs &a, const CUtensorMap &tmA, int kb, cudaStream_t s) {
-  // Resident A only for up to two K blocks: beyond that the streamed
-  // stages fit two CTAs per SM where a resident A tile fits one.
-  const bool stream = kb > 2;
-  if (a.fp8)
-    return stream ? mma_t<KP, true, true>(a, tmA, kb, s) : mma_t<KP, false, true>(a, tmA, kb, s);
-  return stream ? mma_t<KP, true, false>(a, tmA, kb, s) : mma_t<KP, false, false>(a, tmA, kb, s);
+  return a.fp8 ? mma_shaped<KP, true>(a, tmA, kb, s) : mma_shaped<KP, false>(a, tmA, kb, s);
 }
 
 }  // namespace

@@ -486,7 +486,7 @@ drpt_status query_tile(const QueryArgs &a, unsigned max_items, cudaStream_t s) {
 // Queries per item of the grouped form; 0: the few-queries form.  The grouped
 // form stages a leaf once for the queries that fall in it (nq / nleaf on
 // average), the other one reads it for each query.
-constexpr int kQueryWide = 24, kQueryGroup = 2;
+constexpr int kQueryWide = 24, kQueryGroup = 4;
 int query_group(int64_t nq, int nleaf) {
   const int64_t per = nq / nleaf;
   return per >= kQueryWide ? 64 : (per >= kQueryGroup ? 16 : 0);
