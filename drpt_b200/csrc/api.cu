@@ -1155,7 +1155,7 @@ drpt_status run_fp32_leaf(drpt_ctx *c, const drpt_build_desc *desc, const void *
   DRPT_TRY(ws_get(c, "cand_dist", (size_t)n * T * nn, &cdist));
   LeafKnnArgs ka{X, desc->dtype, n, d, T, nn, order, goff, nleaf, cidx, cdist};
   DRPT_TRY(launch_leaf_knn_exact(ka, s));
-  c->launches += leaf_knn_exact_kernels();
+  c->launches += leaf_knn_exact_kernels(ka.k);
   DRPT_CUDA(cudaEventRecord(ev[4], s));
   DRPT_TRY(launch_merge(cidx, cdist, n, T, nn, nn, oi, od, s));
   c->launches += 1;
@@ -1407,7 +1407,7 @@ drpt_status batch_enqueue(drpt_ctx *c, const BatchPlan &bp, const void *X, int32
     if (timed) DRPT_CUDA(cudaEventRecord(c->ev[3], s));
     LeafKnnArgs ka{X, bp.dtype, n, bp.d, T, bp.nn, bp.order, bp.goff, bp.nleaf, bp.cidx, bp.cdist};
     DRPT_TRY(launch_leaf_knn_exact(ka, s));
-    c->launches += leaf_knn_exact_kernels();
+    c->launches += leaf_knn_exact_kernels(ka.k);
     if (timed) DRPT_CUDA(cudaEventRecord(c->ev[4], s));
     DRPT_TRY(launch_merge(bp.cidx, bp.cdist, n, T, bp.nn, bp.nn, oi, od, s));
     c->launches += 1;
@@ -1796,7 +1796,7 @@ static drpt_status build_graph_impl(drpt_ctx *c, const drpt_build_desc *desc, co
   DRPT_TRY(ws_get(c, "cand_dist", (size_t)n * T * nn, &cdist));
   LeafKnnArgs ka{X, desc->dtype, n, d, T, nn, forder, foff, n_final, cidx, cdist};
   DRPT_TRY(launch_leaf_knn_exact(ka, s));
-  c->launches += leaf_knn_exact_kernels();
+  c->launches += leaf_knn_exact_kernels(ka.k);
   DRPT_CUDA(cudaEventRecord(ev[4], s));
 
   // K7: merge into the output.

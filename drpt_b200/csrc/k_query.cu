@@ -18,6 +18,7 @@
 
 #include "kernels.cuh"
 #include "sm100.cuh"
+#include "warp_list.cuh"
 
 namespace drpt {
 namespace {
@@ -38,29 +39,6 @@ __global__ void k_descend(const float *__restrict__ Pq, int64_t nq, int T, int g
   leaf[e] = node - (nleaf - 1);
 }
 
-__device__ __forceinline__ bool qbefore(float da, int32_t ia, float db, int32_t ib) {
-  return da < db || (da == db && (uint32_t)ia < (uint32_t)ib);
-}
-
-// Bitonic sort of 32 (d, id) pairs held one per lane, ascending.
-__device__ __forceinline__ void warp_sort32(float &d, int32_t &id, int lane) {
-#pragma unroll
-  for (int size = 2; size <= 32; size <<= 1)
-#pragma unroll
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      const float od = __shfl_xor_sync(kFull, d, stride);
-      const int32_t oi = __shfl_xor_sync(kFull, id, stride);
-      const bool up = (lane & size) == 0 || size == 32;
-      const bool lower = (lane & stride) == 0;
-      const bool mine_first = qbefore(d, id, od, oi);
-      const bool keep = (lower == up) ? mine_first : !mine_first;
-      if (!keep) {
-        d = od;
-        id = oi;
-      }
-    }
-}
-
 template <typename T>
 __device__ __forceinline__ float4 ld4(const T *p);
 template <>
@@ -71,65 +49,6 @@ template <>
 __device__ __forceinline__ float4 ld4<uint8_t>(const uint8_t *p) {
   const uchar4 v = __ldg(reinterpret_cast<const uchar4 *>(p));
   return make_float4(v.x, v.y, v.z, v.w);
-}
-
-// L (sorted over the lanes) <- the 32 smallest of L and a sorted batch: the
-// minimum of L and the reversed batch is bitonic; a bitonic clean sorts it.
-__device__ __forceinline__ void warp_merge32(float &ld, int32_t &li, float d, int32_t id,
-                                             int lane) {
-  const float rd = __shfl_sync(kFull, d, 31 - lane);
-  const int32_t ri = __shfl_sync(kFull, id, 31 - lane);
-  if (qbefore(rd, ri, ld, li)) {
-    ld = rd;
-    li = ri;
-  }
-#pragma unroll
-  for (int stride = 16; stride > 0; stride >>= 1) {
-    const float od = __shfl_xor_sync(kFull, ld, stride);
-    const int32_t oi = __shfl_xor_sync(kFull, li, stride);
-    const bool lower = (lane & stride) == 0;
-    const bool mine_first = qbefore(ld, li, od, oi);
-    if (lower != mine_first) {
-      ld = od;
-      li = oi;
-    }
-  }
-}
-
-// The warp's sorted list <- its 32 smallest with this lane's candidate
-// (id < 0: none).  Only candidates before the list's k-th entry enter; a few
-// are inserted one by one (a ballot and a shift each), more are sorted and
-// merged as a batch.  Every lane takes part in every shuffle.
-__device__ __forceinline__ void warp_take(float &ld, int32_t &li, float d, int32_t id, int k,
-                                          int lane) {
-  const float kd = __shfl_sync(kFull, ld, k - 1);
-  const int32_t ki = __shfl_sync(kFull, li, k - 1);
-  const bool pass = id >= 0 && qbefore(d, id, kd, ki);
-  unsigned m = __ballot_sync(kFull, pass);
-  if (m == 0) return;
-  if (__popc(m) > 5) {
-    float bd = pass ? d : __int_as_float(0x7f800000);
-    int32_t bi = pass ? id : -1;
-    warp_sort32(bd, bi, lane);
-    warp_merge32(ld, li, bd, bi, lane);
-    return;
-  }
-  do {
-    const int src = __ffs(m) - 1;
-    m &= m - 1;
-    const float v = __shfl_sync(kFull, d, src);
-    const int32_t i = __shfl_sync(kFull, id, src);
-    const int at = __popc(__ballot_sync(kFull, qbefore(ld, li, v, i)));
-    const float ud = __shfl_up_sync(kFull, ld, 1);
-    const int32_t ui = __shfl_up_sync(kFull, li, 1);
-    if (lane == at) {
-      ld = v;
-      li = i;
-    } else if (lane > at) {
-      ld = ud;
-      li = ui;
-    }
-  } while (m);
 }
 
 // Q2a, few queries: block (e, s) takes share s of the S shares of the
@@ -309,18 +228,20 @@ __global__ void k_query_fill(const int32_t *__restrict__ leaf, const int32_t *__
 // Q2b: one item (<= QT queries of one leaf) against every kMT-member tile of
 // the leaf.  Members and queries are staged in kKc-dimension chunks, dimension
 // major, through two shared buffers (the next chunk is in registers while the
-// current one is used); thread (ty, tx) owns queries ty + 16 i and members
-// 4 tx + j, 64 + 4 tx + j: a packed subtraction and a packed multiply-add take
-// two members at once, each pair's sum running over the dimensions in order as
-// in k_query_few.  Then eight lanes' worth of selection: warp w keeps the
-// lists of queries w QT/8 .. in its lanes.  FP32 issue bounds it: two
-// operations per dimension and pair.  QT = 64 serves buckets that fill it;
-// QT = 16 smaller ones, where 64 would mostly compute padding.
+// current one is used); thread (ty, tx) owns queries QT/16 ty + i and members
+// 4 tx + j, 64 + 4 tx + j; a packed multiply-add takes two members at once,
+// each pair's sum running over the dimensions in order as in k_query_few.
+// Then the selection: warp w keeps the lists of queries w QT/8 .. in its
+// lanes.  FP32 issue bounds it: two operations per dimension and pair.  50,000
+// queries of 262,144 x 128 (6 trees, leaves of 1,024): 38.8 ms with a warp per
+// query reading its leaves, 5.3 ms with QT = 64, 10 ms with QT = 16, which
+// serves leaves with fewer queries (kQueryWide), where 64 would mostly compute
+// padding (4,096 queries: 1.2 against 1.5 ms).
 constexpr int kMT = 128, kKc = 32, kQThreads = 256;
 constexpr int kSPitch = kMT + 4;
 template <int QT>
 constexpr size_t query_smem() {
-  return sizeof(float) * (2 * kKc * kMT + 2 * kKc * QT * 2 + QT * kSPitch) +
+  return sizeof(float) * (2 * kKc * kMT + 2 * kKc * QT + QT * kSPitch) +
          sizeof(int32_t) * (kMT + QT);
 }
 
@@ -335,8 +256,8 @@ __global__ void __launch_bounds__(kQThreads, 2) k_query_tile(
   constexpr int QG = QT * kKc / 4 / kQThreads > 0 ? QT * kKc / 4 / kQThreads : 1;  // query quads
   extern __shared__ __align__(16) float sm[];
   float *Ms = sm;                               // [2][kKc][kMT]
-  float *Qs = Ms + 2 * kKc * kMT;               // [2][kKc][QT][2]: -y twice
-  float *St = Qs + 2 * kKc * QT * 2;            // [QT][kSPitch]
+  float *Qs = Ms + 2 * kKc * kMT;               // [2][kKc][QT]
+  float *St = Qs + 2 * kKc * QT;                // [QT][kSPitch]
   int32_t *cid = reinterpret_cast<int32_t *>(St + QT * kSPitch);  // kMT
   int32_t *qid = cid + kMT;                     // QT
   if ((int)blockIdx.x >= *n_items) return;
@@ -380,11 +301,11 @@ __global__ void __launch_bounds__(kQThreads, 2) k_query_tile(
     for (int i = 0; i < QG; ++i) {
       const int g = tid + i * kQThreads, r = g % QT, c = 4 * (g / QT);
       if (g < QT * (kKc / 4)) {
-        float2 *Q = reinterpret_cast<float2 *>(Qs) + (b * kKc + c) * QT + r;
-        Q[0] = make_float2(-pq[i].x, -pq[i].x);
-        Q[QT] = make_float2(-pq[i].y, -pq[i].y);
-        Q[2 * QT] = make_float2(-pq[i].z, -pq[i].z);
-        Q[3 * QT] = make_float2(-pq[i].w, -pq[i].w);
+        float *Q = Qs + (b * kKc + c) * QT + r;
+        Q[0] = pq[i].x;
+        Q[QT] = pq[i].y;
+        Q[2 * QT] = pq[i].z;
+        Q[3 * QT] = pq[i].w;
       }
     }
   };
@@ -414,22 +335,27 @@ __global__ void __launch_bounds__(kQThreads, 2) k_query_tile(
       if (more) fetch(row, k0 + kKc);
       else if (m0 + kMT < m) fetch(next, 0);
       const float *M = Ms + cur * kKc * kMT;
-      const float2 *Q = reinterpret_cast<const float2 *>(Qs) + cur * kKc * QT;
+      const float *Q = Qs + cur * kKc * QT + QPT * ty;
 #pragma unroll 8
       for (int kk = 0; kk < kKc; ++kk) {
         const float4 a = *reinterpret_cast<const float4 *>(M + kk * kMT + 4 * tx);
         const float4 b = *reinterpret_cast<const float4 *>(M + kk * kMT + 64 + 4 * tx);
-        const float2 x[4] = {make_float2(a.x, a.y), make_float2(a.z, a.w),
-                             make_float2(b.x, b.y), make_float2(b.z, b.w)};
+        const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        float y[QPT];
+        if constexpr (QPT == 4) {
+          const float4 q = *reinterpret_cast<const float4 *>(Q + kk * QT);
+          y[0] = q.x; y[1] = q.y; y[2] = q.z; y[3] = q.w;
+        } else {
 #pragma unroll
-        for (int i = 0; i < QPT; ++i) {
-          const float2 y = Q[kk * QT + ty + 16 * i];
+          for (int i = 0; i < QPT; ++i) y[i] = Q[kk * QT + i];
+        }
+#pragma unroll
+        for (int i = 0; i < QPT; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const float2 df = sm100::add2(x[j], y);
+            const float2 df = make_float2(x[2 * j] - y[i], x[2 * j + 1] - y[i]);
             acc[i][j] = sm100::fma2(df, df, acc[i][j]);
           }
-        }
       }
       // the other buffer was last read before the barrier that ended the
       // previous chunk
@@ -440,7 +366,7 @@ __global__ void __launch_bounds__(kQThreads, 2) k_query_tile(
     }
 #pragma unroll
     for (int i = 0; i < QPT; ++i) {
-      float *s = St + (ty + 16 * i) * kSPitch;
+      float *s = St + (QPT * ty + i) * kSPitch;
       *reinterpret_cast<float4 *>(s + 4 * tx) =
           make_float4(sqrtf(acc[i][0].x), sqrtf(acc[i][0].y), sqrtf(acc[i][1].x),
                       sqrtf(acc[i][1].y));
@@ -485,7 +411,11 @@ drpt_status query_tile(const QueryArgs &a, unsigned max_items, cudaStream_t s) {
 
 // Queries per item of the grouped form; 0: the few-queries form.  The grouped
 // form stages a leaf once for the queries that fall in it (nq / nleaf on
-// average), the other one reads it for each query.
+// average), the other one reads it for each query.  262,144 x 128, 256 leaves
+// a tree: 512 queries (2 a leaf) take 0.46 ms with a leaf read per query and
+// 0.75 grouped, 1,024 queries 0.84 and 0.86, 2,048 queries 1.6 and 0.88; with
+// 64 instead of 16 an item 4,096 queries (16 a leaf) 1.5 against 1.2 ms, 8,192
+// queries 1.6 against 2.0.
 constexpr int kQueryWide = 24, kQueryGroup = 4;
 int query_group(int64_t nq, int nleaf) {
   const int64_t per = nq / nleaf;

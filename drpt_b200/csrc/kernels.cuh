@@ -85,7 +85,9 @@ struct LeafKnnArgs {
   float *cand_dist;            // n x T x k
 };
 drpt_status launch_leaf_knn_exact(const LeafKnnArgs &a, cudaStream_t s);
-int leaf_knn_exact_kernels();
+int leaf_knn_exact_kernels(int k);
+// The leaves of more than `above` points (k <= 32; k_fp32gram.cu).
+drpt_status launch_leaf_tiles_exact(const LeafKnnArgs &a, int above, cudaStream_t s);
 
 // ---- K7: cross-tree merge (k_merge.cu) -------------------------------------
 // T sorted lists of `lk` entries per point (n x T x lk) -> the k best distinct.

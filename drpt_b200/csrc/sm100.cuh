@@ -162,6 +162,9 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 }
 
 // (a.x + b.x, a.y + b.y), each lane rounded once: one packed FP32x2 addition.
+// (A packed product followed by this is fused into one multiply-add by the
+// assembler, whatever the rounding modifiers and -fmad say, so where two
+// roundings are wanted the products are scalar.)
 __device__ __forceinline__ float2 add2(float2 a, float2 b) {
   float2 d;
   asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
