@@ -266,10 +266,13 @@ drpt_status global_trees(drpt_ctx *c, const float *P, int64_t n, int T, int gd, 
   const int64_t Gmax = (int64_t)T << last;
   const int64_t Umax = tree_level_max_units(n, T, last);
   TreeLevelArgs a{};
-  DRPT_TRY(ws_get(c, "lv_node_ubase", Gmax + 1, &a.node_ubase));
-  DRPT_TRY(ws_get(c, "lv_unit_node", Umax, &a.unit_node));
-  DRPT_TRY(ws_get(c, "lv_unit_lo", Umax, &a.unit_lo));
-  DRPT_TRY(ws_get(c, "lv_n_units", 1, &a.n_units));
+  a.max_nodes = Gmax;
+  a.max_units = Umax;
+  DRPT_TRY(ws_get(c, "lv_node_ubase", 2 * Gmax, &a.node_ubase));
+  DRPT_TRY(ws_get(c, "lv_unit_node", 2 * Umax, &a.unit_node));
+  DRPT_TRY(ws_get(c, "lv_unit_lo", 2 * Umax, &a.unit_lo));
+  DRPT_TRY(ws_get(c, "lv_n_units", 2 * T, &a.n_units));
+  DRPT_TRY(ws_get(c, "lv_tickets", Gmax, &a.tickets));
   DRPT_TRY(ws_get(c, "lv_node_D", Gmax * kBins, &a.node_D));
   DRPT_TRY(ws_get(c, "lv_unit_s", 2 * Umax, &a.unit_s));
   DRPT_TRY(ws_get(c, "lv_unit_hist", Umax * kBins, &a.unit_hist));
@@ -292,8 +295,7 @@ drpt_status global_trees(drpt_ctx *c, const float *P, int64_t n, int T, int gd, 
     a.off_out = off[cur ^ 1];
     a.medians = medians;
     a.exact = exact;
-    DRPT_TRY(launch_tree_level(a, tree_level_max_units(n, T, level), s));
-    c->launches += tree_level_kernels(exact);
+    DRPT_TRY(launch_tree_level(a, level == 0, level + 2 == gd, s, &c->launches));
     cur ^= 1;
   }
   *order_out = ord[cur];
@@ -510,10 +512,11 @@ drpt_status mixed_leaf_phase(drpt_ctx *c, const void *X, int dtype, int64_t n, i
   st.Xb = xb;
   st.nrm = nrm;
   st.scl = scl;
-  const size_t tiles = (size_t)ceil_div(n, 64) + nleaf;  // the FP32 form's 64-row tiles
-  DRPT_TRY(ws_get(c, "mx_tile_leaf", tiles, &a.tile_leaf));
-  DRPT_TRY(ws_get(c, "mx_tile_r0", tiles, &a.tile_r0));
-  DRPT_TRY(ws_get(c, "mx_n_tiles", 1, &a.n_tiles));
+  const int64_t max_tiles = mixed_max_tiles(n, nleaf);
+  int4 *tiles;
+  int32_t *n_tiles;
+  DRPT_TRY(ws_get(c, "mx_tiles", (size_t)T * max_tiles, &tiles));
+  DRPT_TRY(ws_get(c, "mx_n_tiles", (size_t)T, &n_tiles));
   DRPT_TRY(ws_get(c, "mx_err", 1, &a.err));
   DRPT_TRY(ws_get(c, "mx_run_idx", (size_t)n * kp, &a.cand_idx));
   DRPT_TRY(ws_get(c, "mx_run_dist", (size_t)n * kp, &a.cand_dist));
@@ -538,8 +541,10 @@ drpt_status mixed_leaf_phase(drpt_ctx *c, const void *X, int dtype, int64_t n, i
     return DRPT_OK;
   };
   int e0 = 0, e1 = 0;
+  if (timed) DRPT_TRY(mark(&e0));
+  DRPT_TRY(launch_tile_plan(goff, n, T, nleaf, tiles, n_tiles, s));
+  c->launches += 1;
   if (f32gram) {
-    if (timed) DRPT_TRY(mark(&e0));
     DRPT_TRY(launch_row_norms(X, dtype, n, d, nrm, s));
     c->launches += 1;
     if (timed) {
@@ -551,22 +556,22 @@ drpt_status mixed_leaf_phase(drpt_ctx *c, const void *X, int dtype, int64_t n, i
       a.tree = t;
       a.order = order + (size_t)t * n;
       a.goff = goff + (size_t)t * (nleaf + 1);
-      if (timed) DRPT_TRY(mark(&e0));
+      a.tiles = tiles + t * max_tiles;
+      a.n_tiles = n_tiles + t;
       DRPT_TRY(launch_leaf_f32(a, nrm, s));
-      c->launches += t > 0 ? 3 : 2;  // tile plan, leaf kernel, fold
-      if (timed) {
-        DRPT_TRY(mark(&e1));
-        c->tmma.push_back({e0, e1});
-      }
+      c->launches += t > 0 ? 2 : 1;  // leaf kernel, fold
     }
-    if (timed) DRPT_CUDA(cudaEventRecord(ev[4], s));
+    if (timed) {
+      DRPT_TRY(mark(&e0));
+      c->tmma.push_back({e1, e0});
+      DRPT_CUDA(cudaEventRecord(ev[4], s));
+    }
     DRPT_TRY(launch_rerank(X, dtype, d, order + (size_t)(T - 1) * n, n, a.cand_idx, kp, nn, oi,
                            od, s));
     c->launches += 1;
     if (timed) DRPT_CUDA(cudaEventRecord(ev[5], s));
     return DRPT_OK;
   }
-  if (timed) DRPT_TRY(mark(&e0));
   DRPT_TRY(launch_leaf_means(st, s));
   c->launches += 2;
   if (timed) {
@@ -590,13 +595,14 @@ drpt_status mixed_leaf_phase(drpt_ctx *c, const void *X, int dtype, int64_t n, i
       a.Xb = xb + (size_t)(t - t0) * n * row_bytes;
       a.nrm = nrm + (size_t)(t - t0) * n;
       a.scl = fp8 ? scl + (size_t)(t - t0) * n : scl;
-      if (timed) DRPT_TRY(mark(&e0));
+      a.tiles = tiles + t * max_tiles;
+      a.n_tiles = n_tiles + t;
       DRPT_TRY(launch_leaf_mma(a, s));
-      c->launches += t > 0 ? 3 : 2;  // tile plan, leaf kernel, fold
-      if (timed) {
-        DRPT_TRY(mark(&e1));
-        c->tmma.push_back({e0, e1});
-      }
+      c->launches += t > 0 ? 2 : 1;  // leaf kernel, fold
+    }
+    if (timed) {  // one span for the chunk's trees
+      DRPT_TRY(mark(&e0));
+      c->tmma.push_back({e1, e0});
     }
   }
   if (timed) DRPT_CUDA(cudaEventRecord(ev[4], s));
@@ -830,10 +836,13 @@ drpt_status learn_and_project(drpt_ctx *c, const void *X, int dtype, int64_t n, 
   if (levels >= 2) {
     const int last = levels - 2;
     const int64_t Gmax = (int64_t)T << last, Umax = tree_level_max_units(S, T, last);
-    DRPT_TRY(ws_get(c, "ls_node_ubase", Gmax + 1, &lv.node_ubase));
-    DRPT_TRY(ws_get(c, "ls_unit_node", Umax, &lv.unit_node));
-    DRPT_TRY(ws_get(c, "ls_unit_lo", Umax, &lv.unit_lo));
-    DRPT_TRY(ws_get(c, "ls_n_units", 1, &lv.n_units));
+    lv.max_nodes = Gmax;
+  lv.max_units = Umax;
+  DRPT_TRY(ws_get(c, "ls_node_ubase", 2 * Gmax, &lv.node_ubase));
+    DRPT_TRY(ws_get(c, "ls_unit_node", 2 * Umax, &lv.unit_node));
+    DRPT_TRY(ws_get(c, "ls_unit_lo", 2 * Umax, &lv.unit_lo));
+    DRPT_TRY(ws_get(c, "ls_n_units", 2 * T, &lv.n_units));
+  DRPT_TRY(ws_get(c, "ls_tickets", Gmax, &lv.tickets));
     DRPT_TRY(ws_get(c, "ls_node_D", Gmax * kBins, &lv.node_D));
     DRPT_TRY(ws_get(c, "ls_unit_s", 2 * Umax, &lv.unit_s));
     DRPT_TRY(ws_get(c, "ls_unit_hist", Umax * kBins, &lv.unit_hist));
@@ -894,9 +903,9 @@ drpt_status learn_and_project(drpt_ctx *c, const void *X, int dtype, int64_t n, 
       t.medians = nullptr;
       t.exact = 0;
       t.stop = nullptr;
-      DRPT_TRY(launch_tree_level(t, tree_level_max_units(S, T, l), s));
+      DRPT_TRY(launch_tree_level(t, /*first=*/true, /*last=*/true, s, &c->launches));
       DRPT_TRY(launch_node_label(perm[cur ^ 1], noff[cur ^ 1], 2 * nodes, S, T, node_of, s));
-      c->launches += tree_level_kernels(0) + 2;
+      c->launches += 2;
       cur ^= 1;
     }
   }
@@ -1312,10 +1321,13 @@ drpt_status batch_prepare(drpt_ctx *c, const drpt_batch_desc *desc, const int64_
   const int64_t Gmax = (int64_t)T << last;
   const int64_t Umax = tree_level_max_units(n, T, last);
   TreeLevelArgs &a = bp->lv;
-  DRPT_TRY(ws_get(c, "lv_node_ubase", Gmax + 1, &a.node_ubase));
-  DRPT_TRY(ws_get(c, "lv_unit_node", Umax, &a.unit_node));
-  DRPT_TRY(ws_get(c, "lv_unit_lo", Umax, &a.unit_lo));
-  DRPT_TRY(ws_get(c, "lv_n_units", 1, &a.n_units));
+  a.max_nodes = Gmax;
+  a.max_units = Umax;
+  DRPT_TRY(ws_get(c, "lv_node_ubase", 2 * Gmax, &a.node_ubase));
+  DRPT_TRY(ws_get(c, "lv_unit_node", 2 * Umax, &a.unit_node));
+  DRPT_TRY(ws_get(c, "lv_unit_lo", 2 * Umax, &a.unit_lo));
+  DRPT_TRY(ws_get(c, "lv_n_units", 2 * T, &a.n_units));
+  DRPT_TRY(ws_get(c, "lv_tickets", Gmax, &a.tickets));
   DRPT_TRY(ws_get(c, "lv_node_D", Gmax * kBins, &a.node_D));
   DRPT_TRY(ws_get(c, "lv_unit_s", 2 * Umax, &a.unit_s));
   DRPT_TRY(ws_get(c, "lv_unit_hist", Umax * kBins, &a.unit_hist));
@@ -1325,7 +1337,6 @@ drpt_status batch_prepare(drpt_ctx *c, const drpt_batch_desc *desc, const int64_
   DRPT_TRY(ws_get(c, "lv_node_nleft", Gmax, &a.node_nleft));
   if (bp->mode == DRPT_MODE_MIXED) {
     const int d_pad = mixed_d_pad(d, bp->fp8), kp = bp->kp;
-    const size_t tiles = (size_t)ceil_div(n, 128) + bp->nleaf;
     uint8_t *u8p;
     int32_t *i32p;
     float *f32p;
@@ -1337,9 +1348,9 @@ drpt_status batch_prepare(drpt_ctx *c, const drpt_batch_desc *desc, const int64_
     DRPT_TRY(ws_get(c, "mx_pos", (size_t)T * n, &i32p));
     DRPT_TRY(ws_get(c, "mx_lf", (size_t)T * n, &i32p));
     DRPT_TRY(ws_get(c, "mx_mu", (size_t)T * bp->nleaf * d, &f32p));
-    DRPT_TRY(ws_get(c, "mx_tile_leaf", tiles, &i32p));
-    DRPT_TRY(ws_get(c, "mx_tile_r0", tiles, &i32p));
-    DRPT_TRY(ws_get(c, "mx_n_tiles", 1, &i32p));
+    int4 *i4p;
+    DRPT_TRY(ws_get(c, "mx_tiles", (size_t)T * mixed_max_tiles(n, bp->nleaf), &i4p));
+    DRPT_TRY(ws_get(c, "mx_n_tiles", (size_t)T, &i32p));
     DRPT_TRY(ws_get(c, "mx_err", 1, &ip));
     DRPT_TRY(ws_get(c, "mx_run_idx", (size_t)n * kp, &i32p));
     DRPT_TRY(ws_get(c, "mx_run_dist", (size_t)n * kp, &f32p));
@@ -1395,8 +1406,7 @@ drpt_status batch_enqueue(drpt_ctx *c, const BatchPlan &bp, const void *X, int32
     a.ord_out = bp.ord[cur ^ 1];
     a.val_out = k + 1 < bp.gdm - 1 ? bp.val[cur ^ 1] : nullptr;
     a.off_out = bp.off[cur ^ 1];
-    DRPT_TRY(launch_tree_level(a, tree_level_max_units(n, T, a.level), s));
-    c->launches += tree_level_kernels(0);
+    DRPT_TRY(launch_tree_level(a, k == 0, k + 2 == bp.gdm, s, &c->launches));
     cur ^= 1;
   }
   if (timed) DRPT_CUDA(cudaEventRecord(c->ev[2], s));

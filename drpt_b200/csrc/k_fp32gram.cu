@@ -161,9 +161,8 @@ __device__ __forceinline__ void pair_shift_in(float *Lv, int32_t *Lc, float v, i
 constexpr int kF32Threads = 128;
 template <typename T, int KP>
 __global__ void __launch_bounds__(kF32Threads, 2) k_leaf_f32(
-    const T *__restrict__ X, int d, const int32_t *__restrict__ goff,
-    const int32_t *__restrict__ order, const float *__restrict__ xnorm,
-    const int32_t *__restrict__ tile_leaf, const int32_t *__restrict__ tile_r0,
+    const T *__restrict__ X, int d, const int32_t *__restrict__ order,
+    const float *__restrict__ xnorm, const int4 *__restrict__ tiles,
     const int32_t *__restrict__ n_tiles, int tree, int32_t *__restrict__ run_idx,
     float *__restrict__ run_dist, int32_t *__restrict__ tree_idx, float *__restrict__ tree_dist,
     int align, int *err) {
@@ -175,8 +174,9 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_leaf_f32(
   int32_t *lc = reinterpret_cast<int32_t *>(lv + KP * kRows);
   const int u = blockIdx.x;
   if (u >= *n_tiles) return;  // uniform for the whole block
-  const int leaf = tile_leaf[u], r0 = tile_r0[u];
-  const int32_t lo = goff[leaf], m = goff[leaf + 1] - lo;
+  const int4 tile = __ldg(tiles + u);
+  const int32_t lo = tile.x, m = tile.y;
+  const int r0 = tile.z;
   if (m > kMaxLeaf) {
     if (threadIdx.x == 0) atomicOr(err, 2);
     return;
@@ -485,10 +485,9 @@ drpt_status f32_launch(const MixedTreeArgs &a, const float *xnorm, unsigned grid
                                  (int)f32_smem<KP>()));
   const int step = sizeof(T) == 1 && a.d % 16 == 0 ? 16 : 8;
   const int align = (uintptr_t)a.X % step == 0 ? step : ((uintptr_t)a.X % 8 == 0 ? 8 : 4);
-  k_leaf_f32<T, KP><<<grid, kF32Threads, f32_smem<KP>(), s>>>((const T *)a.X, a.d, a.goff, a.order, xnorm,
-                                                  a.tile_leaf, a.tile_r0, a.n_tiles, a.tree,
-                                                  a.cand_idx, a.cand_dist, a.tree_idx,
-                                                  a.tree_dist, align, a.err);
+  k_leaf_f32<T, KP><<<grid, kF32Threads, f32_smem<KP>(), s>>>(
+      (const T *)a.X, a.d, a.order, xnorm, a.tiles, a.n_tiles, a.tree, a.cand_idx, a.cand_dist,
+      a.tree_idx, a.tree_dist, align, a.err);
   DRPT_LAUNCH_CHECK();
   return DRPT_OK;
 }
@@ -528,8 +527,7 @@ drpt_status launch_leaf_f32(const MixedTreeArgs &a, const float *xnorm, cudaStre
     set_error("FP32 Gram leaf kernel: d %% 8 == 0 needed (got %d)", a.d);
     return DRPT_ERR_UNSUPPORTED;
   }
-  DRPT_TRY(launch_tile_plan(a.goff, a.nleaf, kRows, a.tile_leaf, a.tile_r0, a.n_tiles, s));
-  const unsigned grid = (unsigned)(ceil_div(a.n, kRows) + a.nleaf);
+  const unsigned grid = (unsigned)mixed_max_tiles(a.n, a.nleaf);
   drpt_status st;
   if (a.kp == 16)
     st = a.dtype == DRPT_DTYPE_U8 ? f32_launch<uint8_t, 16>(a, xnorm, grid, s)

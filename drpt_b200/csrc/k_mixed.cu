@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(256) k_leaf_mean(const T *__restrict__ X, int6
   const int32_t *ord = order + (int64_t)t * n;
   const int32_t *g = goff + (int64_t)t * (nleaf + 1);
   const int32_t lo = g[j], m = g[j + 1] - lo;
+  if (m == 0) return;  // no point reads its centre
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float acc[NCH][4];
 #pragma unroll
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(256) k_leaf_mean(const T *__restrict__ X, int6
   for (int i = threadIdx.x; i < d; i += 256) {
     float s = 0.0f;
     for (int w = 0; w < 8; ++w) s += part[w][i];
-    out[i] = mc > 0 ? s / (float)mc : 0.0f;
+    out[i] = s / (float)mc;
   }
 }
 
@@ -396,47 +397,49 @@ __global__ void __launch_bounds__(256, StageCfg<NCH>::min_blocks) k_leaf_stage(c
 }
 
 // ------------------------------------------------------------------ K9
-// Row tiles of `rows` rows of every leaf, in leaf order.
-__global__ void __launch_bounds__(1024) k_tile_plan(const int32_t *__restrict__ goff, int nleaf,
-                                                    int rows, int32_t *tile_leaf,
-                                                    int32_t *tile_r0, int32_t *n_tiles) {
+// Row tiles of every leaf, a block per tree, kRun consecutive leaves per
+// thread and step.  One launch serves all trees (a launch per tree with one
+// thread per run of leaves took 96 us each for the 32,768 leaf slots of a batch
+// of 64 datasets).
+__global__ void __launch_bounds__(1024) k_tile_plan(const int32_t *__restrict__ goff_all,
+                                                    int nleaf, int64_t max_tiles,
+                                                    int4 *__restrict__ tiles_all,
+                                                    int32_t *__restrict__ n_tiles) {
+  constexpr int kRun = 4;
   __shared__ int warp_tot[32];
-  const int per = (nleaf + 1023) / 1024;
-  const int j0 = threadIdx.x * per;
-  int cnt = 0;
-  for (int i = 0; i < per; ++i)
-    if (j0 + i < nleaf) cnt += (goff[j0 + i + 1] - goff[j0 + i] + rows - 1) / rows;
+  const int32_t *goff = goff_all + (int64_t)blockIdx.x * (nleaf + 1);
+  int4 *tiles = tiles_all + (int64_t)blockIdx.x * max_tiles;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int x = cnt;
+  int carry = 0;
+  for (int j0 = 0; j0 < nleaf; j0 += 1024 * kRun) {
+    const int j1 = j0 + threadIdx.x * kRun;
+    int32_t o[kRun + 1];
+    int cnt = 0;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(kFull, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) warp_tot[w] = x;
-  __syncthreads();
-  if (w == 0) {
-    int v = warp_tot[lane];
+    for (int i = 0; i <= kRun; ++i) o[i] = goff[min(j1 + i, nleaf)];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(kFull, v, o);
-      if (lane >= o) v += y;
+    for (int i = 0; i < kRun; ++i) cnt += (o[i + 1] - o[i] + kTM - 1) / kTM;
+    int x = cnt;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+      const int y = __shfl_up_sync(kFull, x, k);
+      if (lane >= k) x += y;
     }
-    warp_tot[lane] = v;
-  }
-  __syncthreads();
-  int base = x - cnt + (w > 0 ? warp_tot[w - 1] : 0);
-  for (int i = 0; i < per; ++i) {
-    const int j = j0 + i;
-    if (j >= nleaf) break;
-    const int nt = (goff[j + 1] - goff[j] + rows - 1) / rows;
-    for (int q = 0; q < nt; ++q) {
-      tile_leaf[base + q] = j;
-      tile_r0[base + q] = q * rows;
+    if (lane == 31) warp_tot[w] = x;
+    __syncthreads();
+    int base = carry + x - cnt;
+    for (int k = 0; k < 32; ++k) {
+      const int y = warp_tot[k];
+      if (k < w) base += y;
+      carry += y;
     }
-    base += nt;
+#pragma unroll
+    for (int i = 0; i < kRun; ++i)
+      for (int r = 0; r < o[i + 1] - o[i]; r += kTM)
+        tiles[base++] = make_int4(o[i], o[i + 1] - o[i], r, j1 + i);
+    __syncthreads();  // warp_tot is reused by the next step
   }
-  if (threadIdx.x == 1023) *n_tiles = base;
+  if (threadIdx.x == 0) n_tiles[blockIdx.x] = carry;
 }
 
 // ------------------------------------------------------------------ K10
@@ -577,9 +580,8 @@ template <int KP, int SHAPE, bool FP8>
 __global__ void __launch_bounds__(MmaCfg<KP, SHAPE>::threads,
                                   MmaCfg<KP, SHAPE>::min_blocks) k_leaf_mma(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-    const int32_t *__restrict__ goff, const int32_t *__restrict__ order,
-    const float *__restrict__ nrm, const float *__restrict__ scl,
-    const int32_t *__restrict__ tile_leaf, const int32_t *__restrict__ tile_r0,
+    const int32_t *__restrict__ order, const float *__restrict__ nrm,
+    const float *__restrict__ scl, const int4 *__restrict__ tiles,
     const int32_t *__restrict__ n_tiles, int kb, int tree, int32_t *__restrict__ run_idx,
     float *__restrict__ run_dist, int32_t *__restrict__ tree_idx, float *__restrict__ tree_dist,
     int *err) {
@@ -610,8 +612,9 @@ __global__ void __launch_bounds__(MmaCfg<KP, SHAPE>::threads,
   const int u = blockIdx.x;
   if (u >= *n_tiles) return;  // uniform for the whole block
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int leaf = tile_leaf[u], r0 = tile_r0[u];
-  const int32_t lo = goff[leaf], m = goff[leaf + 1] - lo;
+  const int4 tile = __ldg(tiles + u);
+  const int32_t lo = tile.x, m = tile.y;
+  const int r0 = tile.z;
   if (m > kMaxLeaf) {  // the candidate keys address at most kMaxLeaf columns
     if (threadIdx.x == 0) atomicOr(err, 2);
     return;  // uniform for the whole block
@@ -1045,6 +1048,58 @@ __global__ void __launch_bounds__(256) k_fold_lists(const float *__restrict__ tr
   }
 }
 
+// The same with KP lanes per point, the lists' entries one per lane: the same
+// networks exchange over shuffles, so the lists (equal distances included) come
+// out the same.  For few points, where a thread per point leaves most of the
+// GPU idle and its ~2,000 dependent operations set the time (2,003 points, 32
+// entries: 10.5 us, these lanes 3.1); it issues twice the instructions (31,337
+// points, 16 entries: 7.3 us against 5.2), hence kFoldLanes.
+template <int KP>
+__global__ void __launch_bounds__(256) k_fold_lanes(const float *__restrict__ tree_dist,
+                                                    const int32_t *__restrict__ tree_idx,
+                                                    int64_t n, float *__restrict__ run_dist,
+                                                    int32_t *__restrict__ run_idx) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = e < n * KP;  // KP lanes of a point alike
+  const int p = threadIdx.x & (KP - 1);
+  const float inf = __int_as_float(0x7f800000);
+  float rd = live ? __ldcs(tree_dist + e) : inf, od = live ? run_dist[e] : inf;
+  int32_t ri = live ? __ldcs(tree_idx + e) : -1, oi = live ? run_idx[e] : -1;
+  bool dup = false;
+#pragma unroll
+  for (int i = 0; i < KP; ++i) dup |= __shfl_sync(kFull, oi, i, KP) == ri;
+  if (dup && ri >= 0) {
+    ri = -1;
+    rd = inf;
+  }
+  // entry p and its partner p ^ j, ascending (up) or descending
+  auto exchange = [&](float &d, int32_t &id, int j, bool up) {
+    const float q = __shfl_xor_sync(kFull, d, j, KP);
+    const int32_t qi = __shfl_xor_sync(kFull, id, j, KP);
+    const bool low = (p & j) == 0;
+    if (low == up ? q < d : d < q) {
+      d = q;
+      id = qi;
+    }
+  };
+#pragma unroll
+  for (int k = 2; k <= KP; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) exchange(rd, ri, j, (p & k) == 0);
+  const float sv = __shfl_sync(kFull, rd, KP - 1 - p, KP);
+  const int32_t si = __shfl_sync(kFull, ri, KP - 1 - p, KP);
+  if (sv < od) {
+    od = sv;
+    oi = si;
+  }
+#pragma unroll
+  for (int j = KP >> 1; j > 0; j >>= 1) exchange(od, oi, j, true);
+  if (live) {
+    run_dist[e] = od;
+    run_idx[e] = oi;
+  }
+}
+
 // ------------------------------------------------------------------ K11
 // One warp per point.  d <= 256: four candidates at a time, eight lanes
 // each, every lane reading 16-byte pieces of the candidate row (a group reads
@@ -1324,12 +1379,11 @@ drpt_status mma_t(const MixedTreeArgs &a, const CUtensorMap &tmA, int kb, cudaSt
     set_error("mixed leaf kernel: no room for %d K blocks", kb);
     return DRPT_ERR_UNSUPPORTED;
   }
-  const unsigned grid = (unsigned)(ceil_div(a.n, kTM) + a.nleaf);
+  const unsigned grid = (unsigned)mixed_max_tiles(a.n, a.nleaf);
   DRPT_CUDA(cudaFuncSetAttribute(k_leaf_mma<KP, SHAPE, FP8>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_leaf_mma<KP, SHAPE, FP8><<<grid, Cfg::threads, smem, s>>>(
-      tmA, tmB, a.goff, a.order, a.nrm, a.scl, a.tile_leaf, a.tile_r0, a.n_tiles, kb, a.tree,
-      a.cand_idx, a.cand_dist, a.tree_idx, a.tree_dist, a.err);
+      tmA, tmB, a.order, a.nrm, a.scl, a.tiles, a.n_tiles, kb, a.tree, a.cand_idx, a.cand_dist, a.tree_idx, a.tree_dist, a.err);
   DRPT_LAUNCH_CHECK();
   if (a.tree > 0) DRPT_TRY(launch_fold_lists(a, s));
   return DRPT_OK;
@@ -1392,8 +1446,6 @@ drpt_status launch_leaf_mma(const MixedTreeArgs &a, cudaStream_t s) {
     set_error("mixed leaf kernel: padded dimension %d unsupported", a.d_pad);
     return DRPT_ERR_UNSUPPORTED;
   }
-  k_tile_plan<<<1, 1024, 0, s>>>(a.goff, a.nleaf, kTM, a.tile_leaf, a.tile_r0, a.n_tiles);
-  DRPT_LAUNCH_CHECK();
   CUtensorMap tmA;
   DRPT_TRY(make_tmap(&tmA, a.Xb, a.n, a.d_pad, kTM, a.fp8));
   const int kb = a.d_pad * esz / 128;
@@ -1403,23 +1455,26 @@ drpt_status launch_leaf_mma(const MixedTreeArgs &a, cudaStream_t s) {
   return DRPT_ERR_UNSUPPORTED;
 }
 
-drpt_status launch_tile_plan(const int32_t *goff, int nleaf, int rows, int32_t *tile_leaf,
-                             int32_t *tile_r0, int32_t *n_tiles, cudaStream_t s) {
-  k_tile_plan<<<1, 1024, 0, s>>>(goff, nleaf, rows, tile_leaf, tile_r0, n_tiles);
+int64_t mixed_max_tiles(int64_t n, int nleaf) { return ceil_div(n, kTM) + nleaf; }
+
+drpt_status launch_tile_plan(const int32_t *goff, int64_t n, int T, int nleaf, int4 *tiles,
+                             int32_t *n_tiles, cudaStream_t s) {
+  k_tile_plan<<<(unsigned)T, 1024, 0, s>>>(goff, nleaf, mixed_max_tiles(n, nleaf), tiles, n_tiles);
   DRPT_LAUNCH_CHECK();
   return DRPT_OK;
 }
 
+constexpr int64_t kFoldLanes = 1 << 18;  // points x entries
 drpt_status launch_fold_lists(const MixedTreeArgs &a, cudaStream_t s) {
-  const unsigned grid = (unsigned)ceil_div(a.n, 256);
-  if (a.kp == 16)
-    k_fold_lists<16><<<grid, 256, 0, s>>>(a.tree_dist, a.tree_idx, a.n, a.cand_dist, a.cand_idx);
-  else if (a.kp == 32)
-    k_fold_lists<32><<<grid, 256, 0, s>>>(a.tree_dist, a.tree_idx, a.n, a.cand_dist, a.cand_idx);
-  else {
+  if (a.kp != 16 && a.kp != 32) {
     set_error("fold: %d candidates per tree unsupported (16 or 32)", a.kp);
     return DRPT_ERR_UNSUPPORTED;
   }
+  const bool lanes = a.n * a.kp <= kFoldLanes;
+  const unsigned grid = (unsigned)ceil_div(lanes ? a.n * a.kp : a.n, 256);
+  auto kern = a.kp == 16 ? (lanes ? k_fold_lanes<16> : k_fold_lists<16>)
+                         : (lanes ? k_fold_lanes<32> : k_fold_lists<32>);
+  kern<<<grid, 256, 0, s>>>(a.tree_dist, a.tree_idx, a.n, a.cand_dist, a.cand_idx);
   DRPT_LAUNCH_CHECK();
   return DRPT_OK;
 }

@@ -26,6 +26,11 @@ drpt_status launch_project(const void *X, int dtype, int64_t n, int d, const Csc
                            float *P, cudaStream_t s);
 
 // ---- K2-K4: one global-tree level of all trees (k_tree.cu) ---------------
+// The units of a level: unit tables of tree t start at t * stride.
+struct UnitPlan {
+  int32_t *node_ubase = nullptr;  // T x 2^level: a node's first unit within its tree
+  int32_t *unit_node = nullptr, *unit_lo = nullptr, *n_units = nullptr;
+};
 struct TreeLevelArgs {
   const float *P;          // projected columns, (T*(gd-1)) x n
   int64_t n;
@@ -41,11 +46,14 @@ struct TreeLevelArgs {
   int p_level0;            // level that reads P directly (0; a batch's root level)
   const int8_t *stop;      // batches: per root slot of level p_level0, the depth
                            // from which its nodes keep all points; nullptr = none
-  // scratch (G = T * 2^level nodes, U = tree_level_max_units units)
-  int32_t *node_ubase;     // G + 1
-  int32_t *unit_node;      // U
-  int32_t *unit_lo;        // U
-  int32_t *n_units;        // 1
+  // scratch (G = T * 2^level nodes and U = tree_level_max_units units of the
+  // deepest level the scratch serves: max_nodes, max_units)
+  int64_t max_nodes, max_units;
+  int32_t *node_ubase;     // 2G
+  int32_t *unit_node;      // 2U
+  int32_t *unit_lo;        // 2U
+  int32_t *n_units;        // 2T
+  unsigned *tickets;       // G
   float *node_D;           // G x 16
   double *unit_s;          // 2U
   unsigned *unit_hist;     // U x 16
@@ -53,10 +61,16 @@ struct TreeLevelArgs {
   int32_t *unit_left;      // U
   int32_t *unit_lbase;     // U
   int32_t *node_nleft;     // G
+  // set by launch_tree_level
+  int64_t unit_stride, next_stride;
+  int direct, fuse;
+  UnitPlan next;
 };
-drpt_status launch_tree_level(const TreeLevelArgs &a, int64_t max_units, cudaStream_t s);
+// `first`: no launch_tree_level of the level before has planned this one's
+// units; `last`: no level follows.  Adds its kernels to *launches.
+drpt_status launch_tree_level(TreeLevelArgs a, bool first, bool last, cudaStream_t s,
+                              int *launches = nullptr);
 int64_t tree_level_max_units(int64_t n, int T, int level);
-int tree_level_kernels(int exact);
 
 // ---- K5: positional local split (k_local.cu) ------------------------------
 struct LocalArgs {
@@ -108,7 +122,8 @@ struct MixedTreeArgs {
   void *Xb;                  // n x d_pad centred rows in leaf order (BF16 or E4M3)
   float *nrm;                // n, squared norms of the rows the tensor cores see
   float *scl;                // n, per-row E4M3 scales (FP8 only)
-  int32_t *tile_leaf, *tile_r0, *n_tiles;  // n / 128 + nleaf
+  int4 *tiles;               // this tree's row tiles (mixed_max_tiles)
+  int32_t *n_tiles;          // and their number
   int32_t *cand_idx;         // n x kp running list (point ids), updated tree by tree
   float *cand_dist;          // n x kp approximate squared distances, ascending
   int32_t *tree_idx;         // n x kp: this tree's list (trees after the first),
@@ -146,9 +161,11 @@ drpt_status launch_leaf_mma(const MixedTreeArgs &a, cudaStream_t s);
 int project_i8_max_cols();
 drpt_status launch_project_i8(const uint8_t *X, int64_t n, int d, const int8_t *S, int nc,
                               float *P, int *err, cudaStream_t s);
-// Row tiles of `rows` rows of every leaf (tile_leaf, tile_r0, *n_tiles).
-drpt_status launch_tile_plan(const int32_t *goff, int nleaf, int rows, int32_t *tile_leaf,
-                             int32_t *tile_r0, int32_t *n_tiles, cudaStream_t s);
+// Row tiles of 128 rows of every leaf of T trees, in leaf order: {leaf start,
+// leaf size, first row, leaf}; tree t's lie from t * mixed_max_tiles on.
+int64_t mixed_max_tiles(int64_t n, int nleaf);
+drpt_status launch_tile_plan(const int32_t *goff, int64_t n, int T, int nleaf, int4 *tiles,
+                             int32_t *n_tiles, cudaStream_t s);
 // Folds a.tree_idx / a.tree_dist (this tree's lists) into the running list.
 drpt_status launch_fold_lists(const MixedTreeArgs &a, cudaStream_t s);
 // FP32 CUDA-core form of the leaf phase (k_fp32gram.cu): ||x||^2 of every

@@ -26,7 +26,10 @@
 
 namespace {
 
-constexpr size_t kStaticScratchBytes = size_t(64) << 20;  // 64 MiB per device
+// Builds may need up to kBuildBytes besides the unit tables of the next level
+// and the tickets (16 bytes a node and 8 a unit, next to at least 76 and 96).
+constexpr size_t kBuildBytes = size_t(64) << 20;
+constexpr size_t kStaticScratchBytes = size_t(72) << 20;  // 72 MiB per device
 constexpr int kMaxDevices = 64;
 
 }  // namespace
@@ -84,6 +87,7 @@ struct Layout {
   float *val[2];      // T x n each: split values of the next level
   int32_t *off_tmp;   // T x (nleaf + 1): the side that is not `offsets`
   TreeLevelArgs lv;   // per-level scratch, sized for the deepest level
+  size_t tables;      // bytes of the second unit tables and the tickets
 };
 
 size_t carve(unsigned char *base, int64_t n, int T, int gd, Layout *L) {
@@ -98,10 +102,14 @@ size_t carve(unsigned char *base, int64_t n, int T, int gd, Layout *L) {
   const int64_t G = (int64_t)T << last;
   const int64_t U = tree_level_max_units(n, T, last);
   TreeLevelArgs &a = L->lv;
-  a.node_ubase = c.take<int32_t>(G + 1);
-  a.unit_node = c.take<int32_t>(U);
-  a.unit_lo = c.take<int32_t>(U);
-  a.n_units = c.take<int32_t>(1);
+  a.max_nodes = G;
+  a.max_units = U;
+  a.node_ubase = c.take<int32_t>(2 * G);
+  a.unit_node = c.take<int32_t>(2 * U);
+  a.unit_lo = c.take<int32_t>(2 * U);
+  a.n_units = c.take<int32_t>(2 * T);
+  a.tickets = c.take<unsigned>(G);
+  L->tables = 4 * (2 * (size_t)G + 2 * (size_t)U + 2 * (size_t)T);
   a.node_D = c.take<float>(G * kBins);
   a.unit_s = c.take<double>(2 * U);
   a.unit_hist = c.take<unsigned>(U * kBins);
@@ -148,7 +156,7 @@ extern "C" drpt_status drpt_global_trees_noalloc(const float *P, int64_t n, int3
   }
   Layout L{};
   const size_t need = carve(nullptr, n, T, gd, &L);
-  if (need > kStaticScratchBytes) {
+  if (need - L.tables > kBuildBytes || need > kStaticScratchBytes) {
     set_error("drpt_global_trees_noalloc: n=%lld, T=%d, gd=%d needs %zu bytes of scratch; the "
               "static scratch holds %zu (use drpt_global_trees for this size)",
               (long long)n, T, gd, need, kStaticScratchBytes);
@@ -181,7 +189,7 @@ extern "C" drpt_status drpt_global_trees_noalloc(const float *P, int64_t n, int3
     a.off_out = off[cur ^ 1];
     a.medians = medians;
     a.exact = exact;
-    DRPT_TRY(launch_tree_level(a, tree_level_max_units(n, T, level), s));
+    DRPT_TRY(launch_tree_level(a, level == 0, level + 2 == gd, s));
     cur ^= 1;
   }
   return DRPT_OK;

@@ -346,7 +346,7 @@ drpt_status drpt_merge_candidates(drpt_ctx *ctx, const int32_t *cand_idx, const 
  * drpt_global_trees (no context: it runs on the calling thread's current
  * device, which must be the device of P, the outputs and `stream`).
  *
- * Scratch comes from a 64 MiB array that is part of the library's device
+ * Scratch comes from a 72 MiB array that is part of the library's device
  * image (every GPU that loads the library holds it until exit); `order` and
  * `offsets` double as one side of the level ping-pong.  A build needs about
  * 12*T*n bytes plus per-level tables; larger builds are rejected with
