@@ -505,8 +505,7 @@ drpt_status mixed_leaf_phase(drpt_ctx *c, const void *X, int dtype, int64_t n, i
   st.nleaf = nleaf;
   st.T = T;
   if (!f32gram) {
-    DRPT_TRY(ws_get(c, "mx_pos", (size_t)T * n, &st.pos));
-    DRPT_TRY(ws_get(c, "mx_lf", (size_t)T * n, &st.lf));
+    DRPT_TRY(ws_get(c, "mx_place", (size_t)T * n, &st.place));
     DRPT_TRY(ws_get(c, "mx_mu", (size_t)T * nleaf * d, &st.mu));
   }
   st.Xb = xb;
@@ -1345,8 +1344,8 @@ drpt_status batch_prepare(drpt_ctx *c, const drpt_batch_desc *desc, const int64_
     DRPT_TRY(ws_get(c, "mx_xb", (size_t)Tc * n * d_pad * (bp->fp8 ? 1 : 2), &u8p));
     DRPT_TRY(ws_get(c, "mx_nrm", (size_t)Tc * n, &f32p));
     DRPT_TRY(ws_get(c, "mx_scl", bp->fp8 ? (size_t)Tc * n : 1, &f32p));
-    DRPT_TRY(ws_get(c, "mx_pos", (size_t)T * n, &i32p));
-    DRPT_TRY(ws_get(c, "mx_lf", (size_t)T * n, &i32p));
+    int2 *i2p;
+    DRPT_TRY(ws_get(c, "mx_place", (size_t)T * n, &i2p));
     DRPT_TRY(ws_get(c, "mx_mu", (size_t)T * bp->nleaf * d, &f32p));
     int4 *i4p;
     DRPT_TRY(ws_get(c, "mx_tiles", (size_t)T * mixed_max_tiles(n, bp->nleaf), &i4p));

@@ -125,16 +125,14 @@ __device__ __forceinline__ void load4_cs<uint8_t>(const uint8_t *p, float *v) {
 // its position in the tree's leaf order and the leaf.
 __global__ void __launch_bounds__(256) k_leaf_index(const int32_t *__restrict__ order,
                                                     const int32_t *__restrict__ goff, int64_t n,
-                                                    int nleaf, int32_t *__restrict__ pos,
-                                                    int32_t *__restrict__ lf) {
+                                                    int nleaf, int2 *__restrict__ place) {
   const int j = blockIdx.x, t = blockIdx.y;
   const int32_t *o = order + (int64_t)t * n;
   const int32_t *g = goff + (int64_t)t * (nleaf + 1);
   const int32_t lo = g[j], hi = g[j + 1];
   for (int32_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
     const int32_t p = __ldg(o + i);
-    pos[(int64_t)t * n + p] = i;
-    lf[(int64_t)t * n + p] = j;
+    place[(int64_t)t * n + p] = make_int2(i, j);
   }
 }
 
@@ -202,6 +200,11 @@ __global__ void __launch_bounds__(256) k_leaf_mean(const T *__restrict__ X, int6
 // centred on its leaf's mean and stored at its position in tree t's leaf
 // order (slice t of Xq, nrm, scl).  The positions and leaves of RB points
 // and up to 32 / RB trees are loaded by one lane each and broadcast.
+// HBM bounds it at 128 dimensions (rows in, every tree's staged rows out; 1M x
+// 128, 6 trees: 0.50 ms, 4.1 TB/s in rows of 256 bytes), issue and the latency
+// of the centres' reads at wide E4M3 rows.  Visiting the points in a leaf
+// order, so that a block's centres come from L1, measured slower (0.60 ms; 960
+// dimensions in E4M3 11.6 against 11.0).
 //
 // BF16 output: the centred row rounded to BF16 (d_pad elements, zero-padded).
 // E4M3 output (FP8): the centred row divided by its scale
@@ -233,6 +236,14 @@ __device__ __forceinline__ float warp_sum_rows(float *s, int lane) {
   return v;
 }
 
+// h * h + s for an FP16 value h, rounded once to FP32 (sm_100's multiply-add
+// of FP16 factors: no conversion first).
+__device__ __forceinline__ float sq_half(unsigned short h, float s) {
+  float d;
+  asm("fma.rn.f32.f16 %0, %1, %1, %2;" : "=f"(d) : "h"(h), "f"(s));
+  return d;
+}
+
 template <int NCH>
 struct StageCfg {
   static constexpr int rb = NCH <= 2 ? 4 / NCH : 1;           // points per warp step
@@ -242,8 +253,7 @@ struct StageCfg {
 // FULL: d == d_pad == 128 * NCH, so no dimension needs a bounds check.
 template <typename T, int NCH, bool FP8, bool FULL>
 __global__ void __launch_bounds__(256, StageCfg<NCH>::min_blocks) k_leaf_stage(const T *__restrict__ X, int64_t n, int d,
-                                                    int d_pad, const int32_t *__restrict__ pos,
-                                                    const int32_t *__restrict__ lf,
+                                                    int d_pad, const int2 *__restrict__ place,
                                                     const float *__restrict__ mu, int nleaf,
                                                     int tc, void *__restrict__ Xq,
                                                     float *__restrict__ nrm,
@@ -272,8 +282,9 @@ __global__ void __launch_bounds__(256, StageCfg<NCH>::min_blocks) k_leaf_stage(c
         const int tt = tg + lane / RB;
         const int64_t r = r0 + lane % RB;
         if (lane < TG * RB && tt < tc && r < n) {
-          my_pos = __ldg(pos + (int64_t)tt * n + r);
-          my_lf = __ldg(lf + (int64_t)tt * n + r);
+          const int2 pl = __ldg(place + (int64_t)tt * n + r);
+          my_pos = pl.x;
+          my_lf = pl.y;
         }
       }
       const int tend = min(tg + TG, tc);
@@ -303,22 +314,15 @@ __global__ void __launch_bounds__(256, StageCfg<NCH>::min_blocks) k_leaf_stage(c
           float c[NCH][4];
 #pragma unroll
           for (int h = 0; h < NCH; ++h) {
-            const int c0 = h * 128 + 4 * lane;
-            if constexpr (FULL) {
-              // two differences per packed FP32x2 multiply-add (-1 * m + v,
-              // one rounding: the same value as v - m)
+            // two differences per packed FP32x2 multiply-add (-1 * m + v, one
+            // rounding: the same value as v - m); past d both are 0
 #pragma unroll
-              for (int e = 0; e < 4; e += 2) {
-                const float2 r = fma2(make_float2(m4[q][h][e], m4[q][h][e + 1]),
-                                      make_float2(-1.0f, -1.0f),
-                                      make_float2(v[q][h][e], v[q][h][e + 1]));
-                c[h][e] = r.x;
-                c[h][e + 1] = r.y;
-              }
-            } else {
-#pragma unroll
-              for (int e = 0; e < 4; ++e)
-                c[h][e] = c0 + e < d ? v[q][h][e] - m4[q][h][e] : 0.0f;
+            for (int e = 0; e < 4; e += 2) {
+              const float2 r = fma2(make_float2(m4[q][h][e], m4[q][h][e + 1]),
+                                    make_float2(-1.0f, -1.0f),
+                                    make_float2(v[q][h][e], v[q][h][e + 1]));
+              c[h][e] = r.x;
+              c[h][e + 1] = r.y;
             }
           }
           const int64_t orow = (int64_t)t * n + row;
@@ -329,8 +333,8 @@ __global__ void __launch_bounds__(256, StageCfg<NCH>::min_blocks) k_leaf_stage(c
             for (int h = 0; h < NCH; ++h)
 #pragma unroll
               for (int e = 0; e < 4; ++e) amax = fmaxf(amax, fabsf(c[h][e]));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(kFull, amax, o));
+            // (not negative, so ordered as its bits)
+            amax = __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(amax)));
             const float sc = amax > 0.0f ? amax / 448.0f : 1.0f;
             const float inv = amax > 0.0f ? 448.0f / amax : 1.0f;
             uint8_t *dst = static_cast<uint8_t *>(Xq) + orow * d_pad;
@@ -342,12 +346,12 @@ __global__ void __launch_bounds__(256, StageCfg<NCH>::min_blocks) k_leaf_stage(c
                     make_float2(c[h][0] * inv, c[h][1] * inv), __NV_SATFINITE, __NV_E4M3);
                 const __nv_fp8x2_storage_t hi2 = __nv_cvt_float2_to_fp8x2(
                     make_float2(c[h][2] * inv, c[h][3] * inv), __NV_SATFINITE, __NV_E4M3);
-                const float2 a = __half22float2(__nv_cvt_fp8x2_to_halfraw2(lo2, __NV_E4M3));
-                const float2 b = __half22float2(__nv_cvt_fp8x2_to_halfraw2(hi2, __NV_E4M3));
-                sq = fmaf(a.x, a.x, sq);
-                sq = fmaf(a.y, a.y, sq);
-                sq = fmaf(b.x, b.x, sq);
-                sq = fmaf(b.y, b.y, sq);
+                const __half2_raw a = __nv_cvt_fp8x2_to_halfraw2(lo2, __NV_E4M3);
+                const __half2_raw b = __nv_cvt_fp8x2_to_halfraw2(hi2, __NV_E4M3);
+                sq = sq_half(a.x, sq);
+                sq = sq_half(a.y, sq);
+                sq = sq_half(b.x, sq);
+                sq = sq_half(b.y, sq);
                 __stcs(reinterpret_cast<unsigned int *>(dst + c0),
                        (unsigned int)lo2 | ((unsigned int)hi2 << 16));
               }
@@ -1336,7 +1340,7 @@ void stage_t(const LeafStageArgs &a, bool means, cudaStream_t s) {
   const T *X = (const T *)a.X;
   if (means) {
     const dim3 g((unsigned)a.nleaf, (unsigned)a.T);
-    k_leaf_index<<<g, 256, 0, s>>>(a.order, a.goff, a.n, a.nleaf, a.pos, a.lf);
+    k_leaf_index<<<g, 256, 0, s>>>(a.order, a.goff, a.n, a.nleaf, a.place);
     k_leaf_mean<T, NCH><<<g, 256, 0, s>>>(X, a.n, a.d, a.order, a.goff, a.nleaf, a.mu);
     return;
   }
@@ -1356,8 +1360,8 @@ void stage_t(const LeafStageArgs &a, bool means, cudaStream_t s) {
       (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(a.n, 8 * RB), (int64_t)sms * per_sm));
   const int64_t toff = (int64_t)a.t0 * a.n;
   const float *mu = a.mu + (int64_t)a.t0 * a.nleaf * a.d;
-  kern<<<grid, 256, 0, s>>>(X, a.n, a.d, a.d_pad, a.pos + toff, a.lf + toff, mu, a.nleaf, a.tc,
-                            a.Xb, a.nrm, a.scl);
+  kern<<<grid, 256, 0, s>>>(X, a.n, a.d, a.d_pad, a.place + toff, mu, a.nleaf, a.tc, a.Xb, a.nrm,
+                            a.scl);
 }
 
 template <typename T>

@@ -140,7 +140,7 @@ struct LeafStageArgs {
   int d, d_pad, fp8;
   const int32_t *order, *goff;  // every tree: T x n leaf orders, T x (nleaf + 1) starts
   int nleaf, T;
-  int32_t *pos, *lf;            // T x n: each point's row in the tree's leaf order, its leaf
+  int2 *place;                  // T x n: each point's row in the tree's leaf order, its leaf
   float *mu;                    // T x nleaf x d leaf centres
   int t0, tc;                   // the chunk
   void *Xb;                     // tc x n x d_pad centred rows, slice t in tree t0 + t's order
