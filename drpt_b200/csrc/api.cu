@@ -138,39 +138,87 @@ drpt_status geometry(int64_t n, int tree_depth, double ratio, Geometry *g) {
   return DRPT_OK;
 }
 
-// K1 with the CSC of the used columns of B built on the host.
-// `tag` names the workspace buffers of the CSC ("csc": the build's own,
-// which an index keeps).
-drpt_status project_cols(drpt_ctx *c, const void *X, int dtype, int64_t n, int d, const float *B,
-                         int L, const std::vector<int32_t> &cols, float *P, cudaStream_t s,
-                         int *nnz_out = nullptr, const char *tag = "csc") {
-  const int ncols = (int)cols.size();
-  std::vector<int32_t> colptr(ncols + 1, 0), row;
+// The CSC of selected columns of a projection matrix, as it is uploaded:
+// column starts (ncols + 1), rows, values.
+struct HostCsc {
+  std::vector<int32_t> words;
+  int ncols = 0, nnz = 0;
+  const int32_t *colptr() const { return words.data(); }
+  const int32_t *row() const { return words.data() + ncols + 1; }
+  float val(int e) const {
+    float v;
+    std::memcpy(&v, words.data() + ncols + 1 + nnz + e, 4);
+    return v;
+  }
+};
+
+// Columns `cols` (distinct) of the d x L matrix whose nonzeros are `nz`, in
+// row order; `sign`: their signs.
+HostCsc csc_of_nonzeros(const std::vector<Nonzero> &nz, int L, const std::vector<int32_t> &cols,
+                        bool sign) {
+  HostCsc h;
+  h.ncols = (int)cols.size();
+  std::vector<int32_t> slot(L, -1), fill(h.ncols + 1, 0);
+  for (int q = 0; q < h.ncols; ++q) slot[cols[q]] = q;
+  for (const Nonzero &z : nz)
+    if (slot[z.col] >= 0) ++fill[slot[z.col] + 1];
+  for (int q = 0; q < h.ncols; ++q) fill[q + 1] += fill[q];
+  h.nnz = fill[h.ncols];
+  h.words.resize((size_t)h.ncols + 1 + 2 * (size_t)h.nnz);
+  std::copy(fill.begin(), fill.end(), h.words.begin());
+  int32_t *row = h.words.data() + h.ncols + 1, *val = row + h.nnz;
+  for (const Nonzero &z : nz) {
+    const int q = slot[z.col];
+    if (q < 0) continue;
+    const int e = fill[q]++;
+    const float v = sign ? (z.val > 0.0f ? 1.0f : -1.0f) : z.val;
+    row[e] = z.row;
+    std::memcpy(val + e, &v, 4);
+  }
+  return h;
+}
+
+// Columns `cols` of the dense d x L matrix B.
+HostCsc csc_of_matrix(const float *B, int d, int L, const std::vector<int32_t> &cols, bool sign) {
+  HostCsc h;
+  h.ncols = (int)cols.size();
+  std::vector<int32_t> colptr(h.ncols + 1, 0), row;
   std::vector<float> val;
-  for (int q = 0; q < ncols; ++q) {
+  for (int q = 0; q < h.ncols; ++q) {
     for (int k = 0; k < d; ++k) {
       const float b = B[(int64_t)k * L + cols[q]];
       if (b != 0.0f) {
         row.push_back(k);
-        val.push_back(b);
+        val.push_back(!sign ? b : (b > 0.0f ? 1.0f : -1.0f));
       }
     }
     colptr[q + 1] = (int32_t)row.size();
   }
-  int32_t *dcol, *drow;
-  float *dval;
-  const std::string t(tag);
-  DRPT_TRY(ws_get(c, (t + "_colptr").c_str(), colptr.size(), &dcol));
-  DRPT_TRY(ws_get(c, (t + "_row").c_str(), std::max<size_t>(row.size(), 1), &drow));
-  DRPT_TRY(ws_get(c, (t + "_val").c_str(), std::max<size_t>(val.size(), 1), &dval));
-  // Pageable sources: the copies complete before these calls return.
-  DRPT_CUDA(cudaMemcpyAsync(dcol, colptr.data(), colptr.size() * 4, cudaMemcpyHostToDevice, s));
-  if (!row.empty()) {
-    DRPT_CUDA(cudaMemcpyAsync(drow, row.data(), row.size() * 4, cudaMemcpyHostToDevice, s));
-    DRPT_CUDA(cudaMemcpyAsync(dval, val.data(), val.size() * 4, cudaMemcpyHostToDevice, s));
-  }
-  if (nnz_out) *nnz_out = (int)row.size();
-  CscDev csc{dcol, drow, dval, ncols};
+  h.nnz = (int)row.size();
+  h.words = std::move(colptr);
+  h.words.insert(h.words.end(), row.begin(), row.end());
+  h.words.resize(h.words.size() + h.nnz);
+  if (h.nnz) std::memcpy(h.words.data() + h.ncols + 1 + h.nnz, val.data(), (size_t)h.nnz * 4);
+  return h;
+}
+
+// Uploads a CSC into workspace buffer `tag` ("csc": the build's own, which an
+// index keeps).
+drpt_status upload_csc(drpt_ctx *c, const HostCsc &h, const char *tag, CscDev *csc,
+                       cudaStream_t s) {
+  int32_t *p;
+  DRPT_TRY(ws_get(c, tag, h.words.size(), &p));
+  // Pageable source: the copy completes before this call returns.
+  DRPT_CUDA(cudaMemcpyAsync(p, h.words.data(), h.words.size() * 4, cudaMemcpyHostToDevice, s));
+  *csc = CscDev{p, p + h.ncols + 1, reinterpret_cast<float *>(p + h.ncols + 1 + h.nnz), h.ncols};
+  return DRPT_OK;
+}
+
+// K1 on a host CSC.
+drpt_status project_cols(drpt_ctx *c, const void *X, int dtype, int64_t n, int d, const HostCsc &h,
+                         float *P, cudaStream_t s, const char *tag = "csc") {
+  CscDev csc{};
+  DRPT_TRY(upload_csc(c, h, tag, &csc, s));
   DRPT_TRY(launch_project(X, dtype, n, d, csc, P, s));
   c->launches += 1;
   return DRPT_OK;
@@ -179,52 +227,33 @@ drpt_status project_cols(drpt_ctx *c, const void *X, int dtype, int64_t n, int d
 // The sign-matrix projection of u8 rows (K1u, a fast form): S = sign of the
 // projection matrix's selected columns (the same sparsity mask), P = X.S^T
 // exactly in integers on the tensor cores, at most project_i8_max_cols()
-// columns per launch.  Also leaves the signs as the CSC an index keeps
-// (csc_*), so that out-of-sample queries project the same way.
-drpt_status project_sign(drpt_ctx *c, const void *X, int64_t n, int d, const float *B, int L,
-                         const std::vector<int32_t> &cols, float *P, cudaStream_t s,
-                         int *nnz_out = nullptr) {
-  const int ncols = (int)cols.size();
+// columns per launch.  Also leaves the signs as the CSC an index keeps, so
+// that out-of-sample queries project the same way.
+drpt_status project_sign(drpt_ctx *c, const void *X, int64_t n, int d, const HostCsc &h, float *P,
+                         cudaStream_t s) {
+  const int ncols = h.ncols;
   if (d % 16 != 0) {
     set_error("the sign-matrix projection needs d %% 16 == 0 (got %d)", d);
     return DRPT_ERR_UNSUPPORTED;
   }
   const int per = project_i8_max_cols();
-  std::vector<int32_t> colptr(ncols + 1, 0), row;
-  std::vector<float> val;
   const int groups = (ncols + per - 1) / per;
-  std::vector<int8_t> S((size_t)groups * per * d, 0);  // per group: `per` rows of d signs
-  for (int q = 0; q < ncols; ++q) {
-    int8_t *srow = S.data() + ((size_t)(q / per) * per + q % per) * d;
-    for (int k = 0; k < d; ++k) {
-      const float b = B[(int64_t)k * L + cols[q]];
-      if (b != 0.0f) {
-        const int8_t sg = b > 0.0f ? 1 : -1;
-        srow[k] = sg;
-        row.push_back(k);
-        val.push_back((float)sg);
-      }
-    }
-    colptr[q + 1] = (int32_t)row.size();
-  }
-  int32_t *dcol, *drow;
-  float *dval;
+  // per group `per` rows of d signs; of the last one as many as are read (a
+  // multiple of 16)
+  const size_t rows = (size_t)(groups - 1) * per + (ncols - (groups - 1) * per + 15) / 16 * 16;
+  std::vector<int8_t> S(rows * d, 0);
+  for (int q = 0; q < ncols; ++q)
+    for (int e = h.colptr()[q]; e < h.colptr()[q + 1]; ++e)
+      S[(size_t)q * d + h.row()[e]] = h.val(e) > 0.0f ? 1 : -1;
+  CscDev csc{};
   int8_t *dS;
   int *err;
-  DRPT_TRY(ws_get(c, "csc_colptr", colptr.size(), &dcol));
-  DRPT_TRY(ws_get(c, "csc_row", std::max<size_t>(row.size(), 1), &drow));
-  DRPT_TRY(ws_get(c, "csc_val", std::max<size_t>(val.size(), 1), &dval));
+  DRPT_TRY(upload_csc(c, h, "csc", &csc, s));
   DRPT_TRY(ws_get(c, "sgn_S", S.size(), &dS));
   DRPT_TRY(ws_get(c, "sgn_err", 1, &err));
-  // Pageable sources: the copies complete before these calls return.
-  DRPT_CUDA(cudaMemcpyAsync(dcol, colptr.data(), colptr.size() * 4, cudaMemcpyHostToDevice, s));
-  if (!row.empty()) {
-    DRPT_CUDA(cudaMemcpyAsync(drow, row.data(), row.size() * 4, cudaMemcpyHostToDevice, s));
-    DRPT_CUDA(cudaMemcpyAsync(dval, val.data(), val.size() * 4, cudaMemcpyHostToDevice, s));
-  }
+  // Pageable source: the copy completes before this call returns.
   DRPT_CUDA(cudaMemcpyAsync(dS, S.data(), S.size(), cudaMemcpyHostToDevice, s));
   DRPT_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
-  if (nnz_out) *nnz_out = (int)row.size();
   for (int g = 0; g < groups; ++g) {
     const int nc = std::min(per, ncols - g * per);
     DRPT_TRY(launch_project_i8(static_cast<const uint8_t *>(X), n, d, dS + (size_t)g * per * d,
@@ -780,8 +809,8 @@ drpt_status learn_and_project(drpt_ctx *c, const void *X, int dtype, int64_t n, 
     for (int k = 0; k < d; ++k) w[k] = nd(dg);
     float *dkey;
     DRPT_TRY(ws_get(c, "ln_pair_key", (size_t)S, &dkey));
-    DRPT_TRY(project_cols(c, xraw, DRPT_DTYPE_F32, S, d, w.data(), 1, std::vector<int32_t>{0},
-                          dkey, s, nullptr, "ln_pair_csc"));
+    DRPT_TRY(project_cols(c, xraw, DRPT_DTYPE_F32, S, d, csc_of_matrix(w.data(), d, 1, {0}, false),
+                          dkey, s, "ln_pair_csc"));
     std::vector<float> key(S);
     DRPT_CUDA(cudaMemcpyAsync(key.data(), dkey, (size_t)S * 4, cudaMemcpyDeviceToHost, s));
     DRPT_CUDA(cudaStreamSynchronize(s));
@@ -995,8 +1024,8 @@ drpt_status run_mixed(drpt_ctx *c, const drpt_build_desc *desc, const void *X, i
   DRPT_CUDA(cudaEventRecord(ev[1], s));
 
   // trees 0 .. Tr-1 split on random projections, the learned ones on MLP values
-  std::vector<float> B((size_t)d * L);
-  host_projection_matrix(desc->seed, d, L, density, B.data());
+  std::vector<Nonzero> B;
+  host_projection_nonzeros(desc->seed, d, L, density, &B);
   std::vector<int32_t> cols;
   for (int t = 0; t < Tr; ++t)
     for (int l = 0; l + 1 < gd; ++l) cols.push_back(t * gd + l);
@@ -1008,12 +1037,18 @@ drpt_status run_mixed(drpt_ctx *c, const drpt_build_desc *desc, const void *X, i
       set_error("the sign-matrix projection takes u8 rows");
       return DRPT_ERR_UNSUPPORTED;
     }
-    if (!cols.empty()) DRPT_TRY(project_sign(c, X, n, d, B.data(), L, cols, P, s, &nnz));
+    if (!cols.empty()) {
+      const HostCsc h = csc_of_nonzeros(B, L, cols, true);
+      nnz = h.nnz;
+      DRPT_TRY(project_sign(c, X, n, d, h, P, s));
+    }
   } else if (desc->projection != DRPT_PROJECTION_GAUSSIAN) {
     set_error("unknown projection %d", desc->projection);
     return DRPT_ERR_INVALID_ARG;
   } else if (!cols.empty()) {
-    DRPT_TRY(project_cols(c, X, desc->dtype, n, d, B.data(), L, cols, P, s, &nnz));
+    const HostCsc h = csc_of_nonzeros(B, L, cols, false);
+    nnz = h.nnz;
+    DRPT_TRY(project_cols(c, X, desc->dtype, n, d, h, P, s));
   }
   LearnResult lres;
   float ms_learn = 0.0f;
@@ -1054,14 +1089,11 @@ drpt_status run_mixed(drpt_ctx *c, const drpt_build_desc *desc, const void *X, i
     DRPT_TRY(dev_copy(&keep->medians, medians, (size_t)T * std::max(nleaf - 1, 1), s));
     keep->ncols_r = (int)cols.size();
     if (!cols.empty()) {
-      int32_t *dcol, *drow;
-      float *dval;
-      DRPT_TRY(ws_get(c, "csc_colptr", cols.size() + 1, &dcol));
-      DRPT_TRY(ws_get(c, "csc_row", std::max<size_t>(nnz, 1), &drow));
-      DRPT_TRY(ws_get(c, "csc_val", std::max<size_t>(nnz, 1), &dval));
-      DRPT_TRY(dev_copy(&keep->csc_col, dcol, cols.size() + 1, s));
-      DRPT_TRY(dev_copy(&keep->csc_row, drow, (size_t)nnz, s));
-      DRPT_TRY(dev_copy(&keep->csc_val, dval, (size_t)nnz, s));
+      int32_t *csc;  // as upload_csc lays it out
+      DRPT_TRY(ws_get(c, "csc", cols.size() + 1 + 2 * (size_t)nnz, &csc));
+      DRPT_TRY(dev_copy(&keep->csc_col, csc, cols.size() + 1, s));
+      DRPT_TRY(dev_copy(&keep->csc_row, csc + cols.size() + 1, (size_t)nnz, s));
+      DRPT_TRY(dev_copy(&keep->csc_val, csc + cols.size() + 1 + nnz, (size_t)nnz, s));
     }
     if (learned > 0) {
       const size_t M = (size_t)learned * (gd - 1);
@@ -1145,14 +1177,14 @@ drpt_status run_fp32_leaf(drpt_ctx *c, const drpt_build_desc *desc, const void *
   cudaEvent_t *ev = c->ev;
   const int launches0 = c->launches;
   DRPT_CUDA(cudaEventRecord(ev[1], s));
-  std::vector<float> B((size_t)d * L);
-  host_projection_matrix(desc->seed, d, L, density, B.data());
+  std::vector<Nonzero> B;
+  host_projection_nonzeros(desc->seed, d, L, density, &B);
   std::vector<int32_t> cols;
   for (int t = 0; t < T; ++t)
     for (int l = 0; l + 1 < gd; ++l) cols.push_back(t * gd + l);
   float *P = nullptr;
   DRPT_TRY(ws_get(c, "P", std::max<size_t>(cols.size(), 1) * n, &P));
-  if (!cols.empty()) DRPT_TRY(project_cols(c, X, desc->dtype, n, d, B.data(), L, cols, P, s));
+  if (!cols.empty()) DRPT_TRY(project_cols(c, X, desc->dtype, n, d, csc_of_nonzeros(B, L, cols, false), P, s));
   int32_t *order, *goff;
   DRPT_TRY(global_trees(c, P, n, T, gd, 0, nullptr, &order, &goff, s));
   DRPT_CUDA(cudaEventRecord(ev[2], s));
@@ -1267,19 +1299,23 @@ drpt_status batch_prepare(drpt_ctx *c, const drpt_batch_desc *desc, const int64_
     const int g = gds[i], cs = (int)set_of_depth.size();
     set_of_depth[g] = cs;
     const int L = g * T;
-    std::vector<float> B((size_t)d * L);
-    host_projection_matrix(desc->seed, d, L, density, B.data());
+    std::vector<Nonzero> B;
+    host_projection_nonzeros(desc->seed, d, L, density, &B);
+    std::vector<int32_t> used;
+    for (int t = 0; t < T; ++t)
+      for (int l = 0; l + 1 < g; ++l) used.push_back(t * g + l);
+    const HostCsc h = csc_of_nonzeros(B, L, used, false);
     colptr.push_back((int32_t)row.size());
+    int q = 0;
     for (int t = 0; t < T; ++t)
       for (int l = 0; l + 1 < gdm; ++l) {
-        if (l + 1 < g)  // levels the dataset splits on; the others project to 0
-          for (int k = 0; k < d; ++k) {
-            const float b = B[(int64_t)k * L + t * g + l];
-            if (b != 0.0f) {
-              row.push_back(k);
-              val.push_back(b);
-            }
+        if (l + 1 < g) {  // levels the dataset splits on; the others project to 0
+          for (int e = h.colptr()[q]; e < h.colptr()[q + 1]; ++e) {
+            row.push_back(h.row()[e]);
+            val.push_back(h.val(e));
           }
+          ++q;
+        }
         colptr.push_back((int32_t)row.size());
       }
   }
@@ -1754,14 +1790,14 @@ static drpt_status build_graph_impl(drpt_ctx *c, const drpt_build_desc *desc, co
   }
 
   // K1: projection on the columns the global trees split on.
-  std::vector<float> B((size_t)d * L);
-  host_projection_matrix(desc->seed, d, L, density, B.data());
+  std::vector<Nonzero> B;
+  host_projection_nonzeros(desc->seed, d, L, density, &B);
   std::vector<int32_t> cols;
   for (int t = 0; t < T; ++t)
     for (int l = 0; l + 1 < g.gd; ++l) cols.push_back(t * g.gd + l);
   float *P = nullptr;
   DRPT_TRY(ws_get(c, "P", std::max<size_t>(cols.size(), 1) * n, &P));
-  if (!cols.empty()) DRPT_TRY(project_cols(c, X, desc->dtype, n, d, B.data(), L, cols, P, s));
+  if (!cols.empty()) DRPT_TRY(project_cols(c, X, desc->dtype, n, d, csc_of_nonzeros(B, L, cols, false), P, s));
   DRPT_CUDA(cudaEventRecord(ev[1], s));
 
   // K2-K4: global trees.
@@ -2132,7 +2168,8 @@ drpt_status drpt_project(drpt_ctx *c, const void *X, int64_t n, int32_t d, int32
     if (cols_host[q] < 0 || cols_host[q] >= L) return DRPT_ERR_INVALID_ARG;
   DRPT_CUDA(cudaSetDevice(c->device));
   std::vector<int32_t> cols(cols_host, cols_host + ncols);
-  return project_cols(c, X, dtype, n, d, B_host, L, cols, P, (cudaStream_t)stream);
+  return project_cols(c, X, dtype, n, d, csc_of_matrix(B_host, d, L, cols, false), P,
+                      (cudaStream_t)stream);
 }
 
 drpt_status drpt_project_sign(drpt_ctx *c, const uint8_t *X, int64_t n, int32_t d,
@@ -2150,7 +2187,7 @@ drpt_status drpt_project_sign(drpt_ctx *c, const uint8_t *X, int64_t n, int32_t 
   DRPT_CUDA(cudaSetDevice(c->device));
   std::vector<int32_t> cols(cols_host, cols_host + ncols);
   const cudaStream_t s = (cudaStream_t)stream;
-  DRPT_TRY(project_sign(c, X, n, d, B_host, L, cols, P, s));
+  DRPT_TRY(project_sign(c, X, n, d, csc_of_matrix(B_host, d, L, cols, true), P, s));
   int serr = 0;
   DRPT_CUDA(cudaMemcpyAsync(&serr, c->bufs["sgn_err"].p, sizeof(int), cudaMemcpyDeviceToHost, s));
   DRPT_CUDA(cudaStreamSynchronize(s));

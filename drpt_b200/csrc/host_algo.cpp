@@ -4,20 +4,189 @@
 #include <algorithm>
 #include <numeric>
 #include <random>
+#if defined(__SSE2__)
+#include <emmintrin.h>
+#endif
 
 namespace drpt {
 
-void host_projection_matrix(uint32_t seed, int d, int L, float density, float *B) {
-  // Row-major over d rows and L columns; one uniform draw per entry, and a
-  // normal draw only for the entries the uniform draw keeps.
-  std::mt19937 gen(seed);
+namespace {
+
+// std::mt19937's sequence (M. Matsumoto and T. Nishimura, "Mersenne Twister",
+// 1998) made 624 outputs at a time, so that draws above a bound can be passed
+// over many at once; a uniform random bit generator for libstdc++'s
+// distributions.
+class Mt19937 {
+ public:
+  using result_type = std::mt19937::result_type;
+  static constexpr result_type min() { return std::mt19937::min(); }
+  static constexpr result_type max() { return std::mt19937::max(); }
+  Mt19937(uint32_t seed, uint32_t bound) : bound_(bound) {
+    x_[0] = seed;
+    for (uint32_t i = 1; i < kN; ++i) x_[i] = 1812433253u * (x_[i - 1] ^ (x_[i - 1] >> 30)) + i;
+  }
+  result_type operator()() {
+    if (at_ == kN) refill();
+    return out_[at_++];
+  }
+  // Skips draws above the bound, at most `most` of them; the number skipped.
+  int64_t skip_above(int64_t most) {
+    int64_t skipped = 0;
+    while (skipped < most) {
+      if (at_ == kN) refill();
+      // the first marked draw from at_ on
+      int w = at_ >> 6;
+      uint64_t m = low_[w] >> (at_ & 63) << (at_ & 63);
+      while (m == 0 && w < kN / 64) m = low_[++w];
+      const int hit = m ? 64 * w + __builtin_ctzll(m) : kN;
+      const int stop = (int)std::min<int64_t>(hit, at_ + (most - skipped));
+      skipped += stop - at_;
+      at_ = stop;
+      if (stop < kN) break;
+    }
+    return skipped;
+  }
+
+ private:
+  static constexpr int kN = 624, kM = 397;
+  static uint32_t twist(uint32_t hi, uint32_t lo) {
+    const uint32_t y = (hi & 0x80000000u) | (lo & 0x7fffffffu);
+    return (y >> 1) ^ ((0u - (lo & 1u)) & 0x9908b0dfu);
+  }
+  // x_[i] for i in [from, to), each from x_[i + shift] (in place: a step of
+  // four reads nothing that it or a later one writes)
+  void twist_range(int from, int to, int shift) {
+    int i = from;
+#if defined(__SSE2__)
+    const __m128i hi = _mm_set1_epi32(INT32_MIN), lo = _mm_set1_epi32(0x7fffffff);
+    const __m128i one = _mm_set1_epi32(1), mat = _mm_set1_epi32((int32_t)0x9908b0dfu);
+    for (; i + 4 <= to; i += 4) {
+      const __m128i a = load(x_ + i), b = load(x_ + i + 1), c = load(x_ + i + shift);
+      const __m128i y = _mm_or_si128(_mm_and_si128(a, hi), _mm_and_si128(b, lo));
+      const __m128i odd = _mm_cmpeq_epi32(_mm_and_si128(b, one), one);
+      store(x_ + i, _mm_xor_si128(c, _mm_xor_si128(_mm_srli_epi32(y, 1), _mm_and_si128(odd, mat))));
+    }
+#endif
+    for (; i < to; ++i) x_[i] = x_[i + shift] ^ twist(x_[i], x_[i + 1]);
+  }
+  void refill() {
+    twist_range(0, kN - kM, kM);
+    twist_range(kN - kM, kN - 1, kM - kN);
+    x_[kN - 1] = x_[kM - 1] ^ twist(x_[kN - 1], x_[0]);
+    at_ = 0;
+#if defined(__SSE2__)
+    // tempered, and the draws at or below the bound marked
+    const __m128i flip = _mm_set1_epi32(INT32_MIN);  // unsigned order as signed
+    const __m128i bound = _mm_xor_si128(_mm_set1_epi32((int32_t)bound_), flip);
+    const __m128i m1 = _mm_set1_epi32((int32_t)0x9d2c5680u);
+    const __m128i m2 = _mm_set1_epi32((int32_t)0xefc60000u);
+    std::fill(low_, low_ + kN / 64 + 1, 0ull);
+    for (int i = 0; i < kN; i += 4) {
+      __m128i y = load(x_ + i);
+      y = _mm_xor_si128(y, _mm_srli_epi32(y, 11));
+      y = _mm_xor_si128(y, _mm_and_si128(_mm_slli_epi32(y, 7), m1));
+      y = _mm_xor_si128(y, _mm_and_si128(_mm_slli_epi32(y, 15), m2));
+      y = _mm_xor_si128(y, _mm_srli_epi32(y, 18));
+      store(out_ + i, y);
+      const int above =
+          _mm_movemask_ps(_mm_castsi128_ps(_mm_cmpgt_epi32(_mm_xor_si128(y, flip), bound)));
+      low_[i >> 6] |= (uint64_t)(above ^ 15) << (i & 63);
+    }
+#else
+    std::fill(low_, low_ + kN / 64 + 1, 0ull);
+    for (int i = 0; i < kN; ++i) {
+      uint32_t y = x_[i];
+      y ^= y >> 11;
+      y ^= (y << 7) & 0x9d2c5680u;
+      y ^= (y << 15) & 0xefc60000u;
+      out_[i] = y ^ (y >> 18);
+      low_[i >> 6] |= (uint64_t)(out_[i] <= bound_) << (i & 63);
+    }
+#endif
+  }
+#if defined(__SSE2__)
+  static __m128i load(const uint32_t *p) {
+    return _mm_loadu_si128(reinterpret_cast<const __m128i *>(p));
+  }
+  static void store(uint32_t *p, __m128i v) { _mm_storeu_si128(reinterpret_cast<__m128i *>(p), v); }
+#endif
+  uint32_t x_[kN], out_[kN], bound_;
+  uint64_t low_[kN / 64 + 1];  // bit i: draw i lies at or below the bound
+  int at_ = kN;
+};
+
+// A generator that returns one given draw, and counts how often it is asked.
+struct OneDraw {
+  using result_type = std::mt19937::result_type;
+  static constexpr result_type min() { return std::mt19937::min(); }
+  static constexpr result_type max() { return std::mt19937::max(); }
+  result_type operator()() {
+    ++asked;
+    return draw;
+  }
+  uint32_t draw;
+  int asked = 0;
+};
+
+}  // namespace
+
+// Row-major over d rows and L columns; one uniform draw per entry, and a
+// normal draw only for the entries the uniform draw keeps.  The uniform value
+// grows with its draw, so the entries it drops are those whose draw lies above
+// a bound, found by bisection with libstdc++'s own distribution; they are most
+// of the draws, and only looked through.
+void host_projection_nonzeros(uint32_t seed, int d, int L, float density,
+                              std::vector<Nonzero> *out) {
+  out->clear();
   std::uniform_real_distribution<float> keep(0, 1);
   std::normal_distribution<float> gauss(0, 1);
-  for (int r = 0; r < d; ++r)
-    for (int c = 0; c < L; ++c) {
+  auto keeps = [&](uint32_t draw) {
+    OneDraw g{draw};
+    return !(keep(g) > density);
+  };
+  OneDraw probe{0u};
+  keep(probe);
+  const int64_t total = (int64_t)d * L;
+  if (probe.asked != 1) {  // another standard library: entry by entry
+    std::mt19937 gen(seed);
+    for (int64_t e = 0; e < total; ++e) {
       const float u = keep(gen);
-      B[(int64_t)r * L + c] = (u > density) ? 0.0f : gauss(gen);
+      const float v = (u > density) ? 0.0f : gauss(gen);
+      if (v != 0.0f) out->push_back({(int32_t)(e / L), (int32_t)(e % L), v});
     }
+    return;
+  }
+  if (!keeps(0u)) return;
+  uint32_t lo = 0u, hi = 0xffffffffu;  // the largest kept draw lies in [lo, hi]
+  while (lo < hi) {
+    const uint32_t mid = lo + (uint32_t)(((uint64_t)hi - lo + 1) / 2);
+    if (keeps(mid)) lo = mid;
+    else hi = mid - 1;
+  }
+  Mt19937 gen(seed, lo);
+  out->reserve((size_t)((double)total * std::min(1.0, 1.1 * ((double)lo + 1.0) / 4294967296.0)) + 16);
+  int64_t row = 0, col = 0;
+  for (int64_t e = 0; e < total; ++e, ++col) {
+    const int64_t s = gen.skip_above(total - e);
+    e += s;
+    if (e >= total) break;
+    col += s;
+    if (col >= 8 * (int64_t)L) {
+      row += col / L;
+      col %= L;
+    }
+    for (; col >= L; col -= L) ++row;
+    gen();  // the kept entry's uniform draw
+    const float v = gauss(gen);
+    if (v != 0.0f) out->push_back({(int32_t)row, (int32_t)col, v});
+  }
+}
+
+void host_projection_matrix(uint32_t seed, int d, int L, float density, float *B) {
+  std::vector<Nonzero> nz;
+  host_projection_nonzeros(seed, d, L, density, &nz);
+  std::fill(B, B + (int64_t)d * L, 0.0f);
+  for (const Nonzero &z : nz) B[(int64_t)z.row * L + z.col] = z.val;
 }
 
 bool host_local_matrix_is_zero(uint32_t seed, int d, int L) {

@@ -10,7 +10,16 @@
 
 namespace drpt {
 
-// d x L row-major sparse Gaussian matrix (math_operations.cpp:48-76).
+// The nonzeros of the d x L sparse Gaussian matrix (math_operations.cpp:48-76),
+// row after row, columns ascending within a row.
+struct Nonzero {
+  int32_t row, col;
+  float val;
+};
+void host_projection_nonzeros(uint32_t seed, int d, int L, float density,
+                              std::vector<Nonzero> *out);
+
+// The same matrix in full, d x L row-major.
 void host_projection_matrix(uint32_t seed, int d, int L, float density, float *B);
 
 // True when the d x L matrix drawn with `density` = 0 from `seed` is all
