@@ -339,15 +339,37 @@ __device__ float block_chain(const float *__restrict__ v, int64_t n, float mu, f
       const int len = (int)min64(kChainChunk, n - c * kChainChunk);
       const int len4 = len & ~3;
       const float4 *src4 = reinterpret_cast<const float4 *>(src);
-#pragma unroll 8
-      for (int i = 0; i < len4 / 4; ++i) {
-        const float4 q = src4[i];
+      auto add = [&](const float4 &q) {
         s = __fadd_rn(s, q.x);
         s = __fadd_rn(s, q.y);
         s = __fadd_rn(s, q.z);
         s = __fadd_rn(s, q.w);
+      };
+      int i = 0;
+      if (len == kChainChunk) {
+        // two register buffers of 32 values: one loads while the other's are
+        // added, so that the chain waits for nothing but its own additions
+        constexpr int kQ = 8, kGroups = kChainChunk / 4 / kQ;
+        static_assert(kGroups % 2 == 0, "two buffers in turn");
+        float4 q0[kQ], q1[kQ];
+#pragma unroll
+        for (int e = 0; e < kQ; ++e) q0[e] = src4[e];
+#pragma unroll 1
+        for (int g = 0; g < kGroups; g += 2) {
+#pragma unroll
+          for (int e = 0; e < kQ; ++e) q1[e] = src4[(g + 1) * kQ + e];
+#pragma unroll
+          for (int e = 0; e < kQ; ++e) add(q0[e]);
+#pragma unroll
+          for (int e = 0; e < kQ; ++e) q0[e] = src4[min(g + 2, kGroups - 1) * kQ + e];
+#pragma unroll
+          for (int e = 0; e < kQ; ++e) add(q1[e]);
+        }
+        i = len4 / 4;
       }
-      for (int i = len4; i < len; ++i) s = __fadd_rn(s, src[i]);
+#pragma unroll 4
+      for (; i < len4 / 4; ++i) add(src4[i]);
+      for (int e = len4; e < len; ++e) s = __fadd_rn(s, src[e]);
     }
   }
   if (threadIdx.x == 0) *result = s;
