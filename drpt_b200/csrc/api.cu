@@ -65,9 +65,11 @@ struct drpt_index {
   int max_leaf = 0;
   __nv_bfloat16 *w1b = nullptr;
   float *b1 = nullptr, *w2 = nullptr, *b2 = nullptr, *c = nullptr, *inv_sigma = nullptr;
-  // query scratch, one allocation grown on demand
+  // query scratch, one allocation grown on demand; tickets that are 0 between
+  // queries
   uint8_t *scratch = nullptr;
   size_t scratch_bytes = 0;
+  unsigned *tickets = nullptr;
 };
 
 namespace drpt {
@@ -1083,6 +1085,8 @@ drpt_status run_mixed(drpt_ctx *c, const drpt_build_desc *desc, const void *X, i
     const size_t esz = desc->dtype == DRPT_DTYPE_U8 ? 1 : 4;
     DRPT_TRY(dev_copy((uint8_t **)&keep->X, X, (size_t)n * d * esz, s));
     DRPT_TRY(dev_copy(&keep->order, order, (size_t)T * n, s));
+    DRPT_CUDA(cudaMalloc((void **)&keep->tickets, kQueryTickets * sizeof(unsigned)));
+    DRPT_CUDA(cudaMemsetAsync(keep->tickets, 0, kQueryTickets * sizeof(unsigned), s));
     DRPT_TRY(dev_copy(&keep->goff, goff, (size_t)T * (nleaf + 1), s));
     std::vector<int32_t> h((size_t)T * (nleaf + 1));
     DRPT_CUDA(cudaMemcpyAsync(h.data(), goff, h.size() * 4, cudaMemcpyDeviceToHost, s));
@@ -2026,7 +2030,7 @@ static void index_free(drpt_index *x) {
   if (!x) return;
   cudaSetDevice(x->device);
   void *ptrs[] = {x->X, x->order, x->goff, x->medians, x->csc_col, x->csc_row, x->csc_val,
-                  x->w1b, x->b1, x->w2, x->b2, x->c, x->inv_sigma, x->scratch};
+                  x->w1b, x->b1, x->w2, x->b2, x->c, x->inv_sigma, x->scratch, x->tickets};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   delete x;
@@ -2065,7 +2069,7 @@ static drpt_status query_block(drpt_index *x, const void *queries, int64_t nq, i
   const int d = x->d, T = x->T, cols = T * (x->gd - 1);
   const size_t esz = x->dtype == DRPT_DTYPE_U8 ? 1 : 4, pairs = (size_t)nq * T;
   const bool aligned = !on_device || (uintptr_t)queries % (4 * esz) == 0;
-  const QueryPlan p = query_plan(nq, T, x->nleaf, x->max_leaf, k, aligned);
+  const QueryPlan p = query_plan(nq, T, x->nleaf, x->max_leaf, k, aligned, x->Tl == 0);
   // the block's buffers, laid out in one allocation (16-byte aligned parts)
   size_t total = 0;
   auto part = [&](size_t bytes) {
@@ -2097,10 +2101,8 @@ static drpt_status query_block(drpt_index *x, const void *queries, int64_t nq, i
   }
   // the queries' split values: random columns, then the learned MLP outputs
   float *P = (float *)(b + o_P);
-  if (x->ncols_r > 0) {
-    CscDev csc{x->csc_col, x->csc_row, x->csc_val, x->ncols_r};
-    DRPT_TRY(launch_project(Q, x->dtype, nq, d, csc, P, s));
-  }
+  const CscDev csc{x->csc_col, x->csc_row, x->csc_val, x->ncols_r};
+  if (x->ncols_r > 0 && !p.descend) DRPT_TRY(launch_project(Q, x->dtype, nq, d, csc, P, s));
   if (x->Tl > 0) {
     int *err = (int *)(b + o_err);
     __nv_bfloat16 *xb = (__nv_bfloat16 *)(b + o_qxb);
@@ -2112,10 +2114,11 @@ static drpt_status query_block(drpt_index *x, const void *queries, int64_t nq, i
     *err_out = err;
   }
   int32_t *leaf = (int32_t *)(b + o_leaf);
-  DRPT_TRY(launch_descend(P, nq, T, x->gd, x->medians, leaf, s));
+  if (!p.descend) DRPT_TRY(launch_descend(P, nq, T, x->gd, x->medians, leaf, s));
   int32_t *oi = on_device ? out_idx : (int32_t *)(b + o_qi);
   float *od = on_device && out_dist ? out_dist : (float *)(b + o_qd);
-  const QueryArgs a{x->X, x->dtype, d, x->n, Q, nq, T, x->order, x->goff, x->nleaf, leaf, k,
+  const QueryArgs a{x->X, x->dtype, d, x->n, Q, nq, T, x->order, x->goff, x->nleaf, leaf, csc,
+                    x->medians, x->gd, x->tickets, k,
                     (int32_t *)(b + o_ci), (float *)(b + o_cd), (int32_t *)(b + o_rank),
                     (int32_t *)(b + o_cnt), (int32_t *)(b + o_off), (int4 *)(b + o_items),
                     (int32_t *)(b + o_nit), (int32_t *)(b + o_list), oi, od};

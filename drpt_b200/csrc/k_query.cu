@@ -51,35 +51,115 @@ __device__ __forceinline__ float4 ld4<uint8_t>(const uint8_t *p) {
   return make_float4(v.x, v.y, v.z, v.w);
 }
 
-// Q2a, few queries: block (e, s) takes share s of the S shares of the
-// members of query e / T's leaf in tree e % T; warps take 32 members at a
-// time, a lane each.  Latency bounds it (one query: a few thousand members),
-// so the members spread over T * S blocks of eight warps and a lane keeps
-// kBurst 16-byte pieces of its row in flight; a whole leaf per query on one
-// warp took 911 us for one query of 6 trees with 1,024-point leaves.
+// The leaf of a query in tree t, by one warp: lane l sums the query's value of
+// level l (as k_project does: the column's nonzeros in order, each product and
+// sum rounded), then the walk of k_descend, kWalk levels at a time: lanes load
+// the medians of the whole subtree below the node, so that a round of loads
+// serves kWalk steps.
+struct QueryTrees {
+  const int32_t *colptr, *row;  // the trees' columns, T * (gd - 1)
+  const float *val, *medians;   // T x (2^(gd-1) - 1), heap order
+  int gd;
+};
+__device__ __forceinline__ int warp_descend(const QueryTrees &q, int t, const float *qv,
+                                            int lane) {
+  constexpr int kWalk = 5;
+  const int levels = q.gd - 1;
+  const float *med = q.medians + (int64_t)t * ((1 << levels) - 1);
+  float v = 0.0f;
+  if (lane < levels) {
+    const int e0 = __ldg(q.colptr + t * levels + lane), e1 = __ldg(q.colptr + t * levels + lane + 1);
+#pragma unroll 4
+    for (int e = e0; e < e1; ++e) v = __fadd_rn(v, __fmul_rn(qv[__ldg(q.row + e)], __ldg(q.val + e)));
+  }
+  int node = 0;  // heap index; children of h are 2h + 1 (left), 2h + 2 (right)
+  for (int l0 = 0; l0 < levels; l0 += kWalk) {
+    // lane i holds heap node i of the subtree below `node`: depth dl, and the
+    // (i + 1 - 2^dl)-th of that level
+    const int dl = 31 - __clz(lane + 1);
+    const int h = ((node + 1) << dl) - 1 + (lane + 1 - (1 << dl));
+    const float m = dl < kWalk && l0 + dl < levels ? __ldg(med + h) : 0.0f;
+    int at = 0;
+    for (int i = 0; i < kWalk && l0 + i < levels; ++i) {
+      const float x = __shfl_sync(kFull, v, l0 + i), mi = __shfl_sync(kFull, m, at);
+      const int right = x <= mi ? 0 : 1;
+      at = 2 * at + 1 + right;
+      node = 2 * node + 1 + right;
+    }
+  }
+  return node - ((1 << levels) - 1);
+}
+
+// L <- the 32 smallest of L and a list of k entries (sorted over the lanes,
+// lanes from k on ignored) whose members may lie in L already; a member carries
+// the same distance in both, so it is skipped.  `tmp`: 64 words of the warp.
+__device__ __forceinline__ void warp_join(float &ld, int32_t &li, float d, int32_t id, int k,
+                                          int lane, float *tmp) {
+  bool fresh = lane < k && id >= 0;
+  for (int j = 0; j < k; ++j) fresh &= __shfl_sync(kFull, li, j) != id;
+  const unsigned m = __ballot_sync(kFull, fresh);
+  if (m == 0) return;
+  // the fresh entries side by side, still sorted
+  int32_t *ti = reinterpret_cast<int32_t *>(tmp + 32);
+  tmp[lane] = __int_as_float(0x7f800000);
+  ti[lane] = -1;
+  __syncwarp();
+  const int at = __popc(m & ((1u << lane) - 1u));
+  if (fresh) {
+    tmp[at] = d;
+    ti[at] = id;
+  }
+  __syncwarp();
+  warp_merge32(ld, li, tmp[lane], ti[lane], lane);
+  __syncwarp();  // tmp is reused
+}
+
+// Q2a, few queries: block (e, s) takes share s of the S shares of the members
+// of query e / T's leaf in tree e % T; warps take 32 members at a time, a lane
+// each.  Latency bounds it (one query: a few thousand members), so the members
+// spread over T * S blocks of eight warps and a lane keeps kBurst 16-byte
+// pieces of its row in flight; a whole leaf per query on one warp took 911 us
+// for one query of 6 trees with 1,024-point leaves.  With `trees` the block
+// also finds its leaf itself, and with `tickets` (one per query, 0 between
+// calls) the query's last block merges its lists into the result: one launch
+// where four took 26 us of the GPU.
 constexpr int kFewWarps = 8;
 template <typename T>
 __global__ void __launch_bounds__(32 * kFewWarps) k_query_few(
     const T *__restrict__ X, int d, int64_t n, const T *__restrict__ Qx, int T_, int S,
     const int32_t *__restrict__ order, const int32_t *__restrict__ goff, int nleaf,
-    const int32_t *__restrict__ leaf, int k, int32_t *__restrict__ ci, float *__restrict__ cd) {
+    const int32_t *__restrict__ leaf, QueryTrees trees, int k, int32_t *ci, float *cd,
+    unsigned *tickets, int32_t *__restrict__ oi, float *__restrict__ od) {
   constexpr int kBurst = 8;
   extern __shared__ __align__(16) float qv[];  // the query's d values
   __shared__ float sd[kFewWarps][32];
   __shared__ int32_t si[kFewWarps][32];
+  __shared__ int leaf_sh;
+  __shared__ float tmp[kFewWarps][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t e = blockIdx.x / S;
   const int s = (int)(blockIdx.x - e * S);
   const int64_t q = e / T_;
   const int t = (int)(e - q * T_);
   for (int c = threadIdx.x; c < d; c += blockDim.x) qv[c] = (float)Qx[q * d + c];
-  const int lf = __ldg(leaf + e);
+  int lf;
+  if (trees.medians) {
+    __syncthreads();
+    if (warp == 0) {
+      const int l = warp_descend(trees, t, qv, lane);
+      if (lane == 0) leaf_sh = l;
+    }
+    __syncthreads();
+    lf = leaf_sh;
+  } else {
+    lf = __ldg(leaf + e);
+    __syncthreads();
+  }
   const int32_t *go = goff + (int64_t)t * (nleaf + 1);
   const int32_t lo0 = __ldg(go + lf), m = __ldg(go + lf + 1) - lo0;
   const int32_t per = ((m + S - 1) / S + 31) & ~31;
   const int32_t lo = lo0 + min(s * per, m), hi = lo0 + min((s + 1) * per, m);
   const int32_t *ord = order + (int64_t)t * n;
-  __syncthreads();
   const float inf = __int_as_float(0x7f800000);
   float ld = inf;  // the list: lane j holds the j-th best
   int32_t li = -1;
@@ -112,47 +192,52 @@ __global__ void __launch_bounds__(32 * kFewWarps) k_query_few(
   sd[warp][lane] = ld;
   si[warp][lane] = li;
   __syncthreads();
-  if (warp != 0) return;
-  for (int w = 1; w < kFewWarps; ++w) warp_merge32(ld, li, sd[w][lane], si[w][lane], lane);
-  if (lane < k) {
-    ci[(int64_t)blockIdx.x * k + lane] = li;
-    cd[(int64_t)blockIdx.x * k + lane] = ld;
+  if (warp == 0) {
+    for (int w = 1; w < kFewWarps; ++w) warp_merge32(ld, li, sd[w][lane], si[w][lane], lane);
+    if (lane < k) {
+      ci[(int64_t)blockIdx.x * k + lane] = li;
+      cd[(int64_t)blockIdx.x * k + lane] = ld;
+    }
+    if (tickets) {
+      __threadfence();
+      __syncwarp();
+      unsigned old = 0u;
+      if (lane == 0) old = atomicAdd(tickets + q, 1u);
+      old = __shfl_sync(kFull, old, 0);
+      if (lane == 0) {
+        leaf_sh = old == (unsigned)(T_ * S) - 1u;
+        if (leaf_sh) tickets[q] = 0u;  // for the next call
+      }
+      __threadfence();
+    }
   }
-}
-
-// Q3, few queries: one block per query merges its `lists` sorted lists of k
-// entries (the same member from two trees carries the same distance bits, so
-// it counts once); warps take lists in turn, warp 0 joins the warps' lists.
-__device__ __forceinline__ void warp_join(float &ld, int32_t &li, float d, int32_t id, int k,
-                                          int lane) {
-  bool dup = false;
-  for (int j = 0; j < k; ++j) dup |= __shfl_sync(kFull, li, j) == id;
-  if (dup || lane >= k) id = -1;
-  warp_take(ld, li, d, id, k, lane);
-}
-
-__global__ void __launch_bounds__(32 * kFewWarps) k_query_join(const int32_t *__restrict__ ci,
-                                                               const float *__restrict__ cd,
-                                                               int lists, int k,
-                                                               int32_t *__restrict__ oi,
-                                                               float *__restrict__ od) {
-  __shared__ float sd[kFewWarps][32];
-  __shared__ int32_t si[kFewWarps][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t q = blockIdx.x;
-  const float inf = __int_as_float(0x7f800000);
-  float ld = inf;
-  int32_t li = -1;
-  for (int l = warp; l < lists; l += kFewWarps) {
-    const int64_t o = (q * lists + l) * k + lane;
-    warp_join(ld, li, lane < k ? __ldg(cd + o) : inf, lane < k ? __ldg(ci + o) : -1, k, lane);
+  if (!tickets) return;
+  __syncthreads();
+  if (!leaf_sh) return;  // block-uniform
+  // the query's last block: warps take its T * S lists in turn, warp 0 joins
+  // the warps' lists
+  ld = inf;
+  li = -1;
+  const int lists = T_ * S;
+  for (int l0 = warp; l0 < lists; l0 += 4 * kFewWarps) {
+    float d4[4];
+    int32_t i4[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int l = l0 + i * kFewWarps;
+      const bool in = l < lists && lane < k;
+      d4[i] = in ? __ldcg(cd + (q * lists + l) * k + lane) : inf;
+      i4[i] = in ? __ldcg(ci + (q * lists + l) * k + lane) : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) warp_join(ld, li, d4[i], i4[i], k, lane, tmp[warp]);
   }
   sd[warp][lane] = ld;
   si[warp][lane] = li;
   __syncthreads();
   if (warp != 0) return;
   for (int w = 1; w < min(kFewWarps, lists); ++w)
-    warp_join(ld, li, sd[w][lane], si[w][lane], k, lane);
+    warp_join(ld, li, sd[w][lane], si[w][lane], k, lane, tmp[0]);
   if (lane < k) {
     oi[q * k + lane] = li;
     od[q * k + lane] = li >= 0 ? ld : inf;
@@ -336,6 +421,7 @@ __global__ void __launch_bounds__(kQThreads, 2) k_query_tile(
       else if (m0 + kMT < m) fetch(next, 0);
       const float *M = Ms + cur * kKc * kMT;
       const float *Q = Qs + cur * kKc * QT + QPT * ty;
+      if (2 * QPT * warp < nqi)  // a warp of the item's queries (else all padding)
 #pragma unroll 8
       for (int kk = 0; kk < kKc; ++kk) {
         const float4 a = *reinterpret_cast<const float4 *>(M + kk * kMT + 4 * tx);
@@ -423,7 +509,9 @@ int query_group(int64_t nq, int nleaf) {
 }
 
 // Shares that the few-queries form cuts a leaf into: until the pairs fill the
-// SMs, but no share below the block's 256 members.
+// SMs, but no share below the block's 256 members.  (More than one share only
+// below 8 * 148 pairs, so below kQueryTickets queries.)
+static_assert(kQueryTickets >= 8 * 148, "lists of shares are joined by the last block");
 int query_shares(int64_t pairs, int max_leaf) {
   const int most = (int)ceil_div(std::max(max_leaf, 1), 32 * kFewWarps);
   return (int)std::max<int64_t>(1, std::min<int64_t>(most, 8 * 148 / std::max<int64_t>(pairs, 1)));
@@ -440,14 +528,19 @@ drpt_status launch_descend(const float *Pq, int64_t nq, int T, int gd, const flo
 }
 
 // `aligned`: the query rows can be read in 16-byte (u8: 4-byte) pieces, as the
-// grouped form does.
-QueryPlan query_plan(int64_t nq, int T, int nleaf, int max_leaf, int k, bool aligned) {
+// grouped form does.  `random_only`: no tree splits on learned values.
+constexpr int kQueryWalk = 32;
+QueryPlan query_plan(int64_t nq, int T, int nleaf, int max_leaf, int k, bool aligned,
+                     bool random_only) {
   QueryPlan p{};
   p.qt = aligned ? query_group(nq, nleaf) : 0;
   const int64_t pairs = nq * T;
   if (p.qt == 0) {
     p.shares = query_shares(pairs, max_leaf);
     p.lists = pairs * p.shares;
+    // the block's own walk costs each of them about 4 us, two launches 10
+    p.descend = random_only && nq <= kQueryWalk;
+    p.join = nq <= kQueryTickets;
   } else {
     p.shares = 1;
     p.lists = pairs;
@@ -470,20 +563,18 @@ drpt_status launch_query(const QueryArgs &a, const QueryPlan &p, cudaStream_t s)
       set_error("queries: %lld (query, tree) pairs in one launch", (long long)p.lists);
       return DRPT_ERR_UNSUPPORTED;
     }
+    QueryTrees trees{};
+    if (p.descend) trees = QueryTrees{a.csc.colptr, a.csc.row, a.csc.val, a.medians, a.gd};
     auto few = [&](auto *X, auto *Q) {
       using E = std::remove_const_t<std::remove_pointer_t<decltype(X)>>;
       k_query_few<E><<<(unsigned)p.lists, 32 * kFewWarps, a.d * sizeof(float), s>>>(
-          X, a.d, a.n, Q, a.T, p.shares, a.order, a.goff, a.nleaf, a.leaf, a.k, a.ci, a.cd);
+          X, a.d, a.n, Q, a.T, p.shares, a.order, a.goff, a.nleaf, a.leaf, trees, a.k, a.ci, a.cd,
+          p.join ? a.tickets : nullptr, a.oi, a.od);
     };
     if (u8) few((const uint8_t *)a.X, (const uint8_t *)a.Q);
     else few((const float *)a.X, (const float *)a.Q);
     DRPT_LAUNCH_CHECK();
-    if (p.shares > 1) {
-      k_query_join<<<(unsigned)a.nq, 32 * kFewWarps, 0, s>>>(a.ci, a.cd, a.T * p.shares, a.k, a.oi,
-                                                             a.od);
-      DRPT_LAUNCH_CHECK();
-      return DRPT_OK;
-    }
+    if (p.join) return DRPT_OK;
   } else {
     const int64_t pairs = a.nq * a.T;
     const unsigned grid = (unsigned)ceil_div(pairs, 256);

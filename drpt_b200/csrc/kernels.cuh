@@ -188,8 +188,11 @@ drpt_status launch_descend(const float *Pq, int64_t nq, int T, int gd, const flo
 struct QueryPlan {
   int qt, shares;
   int64_t lists, entries, buckets, items;
+  bool descend, join;  // few queries: the leaves found, the lists joined in the same launch
 };
-QueryPlan query_plan(int64_t nq, int T, int nleaf, int max_leaf, int k, bool aligned);
+constexpr int64_t kQueryTickets = 4096;  // queries with a ticket (QueryArgs::tickets)
+QueryPlan query_plan(int64_t nq, int T, int nleaf, int max_leaf, int k, bool aligned,
+                     bool random_only);
 
 struct QueryArgs {
   const void *X;               // n x d indexed rows
@@ -201,7 +204,11 @@ struct QueryArgs {
   int T;
   const int32_t *order, *goff; // T x n, T x (nleaf + 1)
   int nleaf;
-  const int32_t *leaf;         // nq x T
+  const int32_t *leaf;         // nq x T (unused where plan.descend)
+  CscDev csc;                  // the split functions and medians (plan.descend)
+  const float *medians;
+  int gd;
+  unsigned *tickets;           // kQueryTickets, 0 between calls (plan.join)
   int k;
   int32_t *ci;                 // plan.entries
   float *cd;
