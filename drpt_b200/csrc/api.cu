@@ -906,14 +906,14 @@ drpt_status learn_and_project(drpt_ctx *c, const void *X, int dtype, int64_t n, 
       const float bc1 = 1.0f - std::pow(0.9f, (float)(it + 1));
       const float bc2 = 1.0f - std::pow(0.999f, (float)(it + 1));
       DRPT_TRY(launch_learn_step(a, kLearnLr, bc1, bc2, nullptr, s));
-      c->launches += learn_step_kernels();
+      c->launches += learn_step_kernels(true);
       if (it == 0) DRPT_TRY(launch_learn_loss(a, loss, 0, s));
     }
     // the loss and outputs at the trained weights
     DRPT_TRY(launch_learn_step(a, 0.0f, 1.0f, 1.0f, nullptr, s));
     DRPT_TRY(launch_learn_loss(a, loss, 1, s));
     DRPT_TRY(launch_stack(a, d_pad, levels, l, wb, db1, dw2, db2, s));
-    c->launches += learn_step_kernels() + 3;
+    c->launches += learn_step_kernels(false) + 3;
     if (l + 1 < levels) {
       // split every node of the sample at the histogram median of f
       DRPT_TRY(launch_gather_f(a, fp, s));

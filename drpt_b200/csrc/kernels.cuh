@@ -247,7 +247,7 @@ struct LearnArgs {
 };
 drpt_status launch_learn_step(const LearnArgs &a, float lr, float bc1, float bc2, float *grad_out,
                               cudaStream_t s);
-int learn_step_kernels();
+int learn_step_kernels(bool train);  // false: lr 0 and no gradient wanted
 drpt_status launch_learn_init(const LearnArgs &a, uint64_t seed, int level, cudaStream_t s);
 drpt_status launch_learn_pairs(const LearnArgs &a, int *cnt, cudaStream_t s);
 drpt_status launch_learn_loss(const LearnArgs &a, float *acc, int slot, cudaStream_t s);
