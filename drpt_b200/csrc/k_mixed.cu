@@ -1015,25 +1015,74 @@ __global__ void __launch_bounds__(MmaCfg<KP, SHAPE>::threads,
 // KP best distinct candidates of the trees before: neighbours the running
 // list already holds are dropped from the new list, which is re-sorted, and a
 // bitonic merge keeps the KP best by distance.
+//
+// A warp's 32 lists of one array are consecutive: it loads and stores them 512
+// bytes at a time and turns them (a lane's list <-> 32 consecutive 16-byte pieces)
+// through 4 KB of shared memory of its own, 16-byte piece c of point p at c ^ p
+// (c ^ p / 2 with four pieces a point), which uses all banks both ways.  A lane
+// reading its own 128-byte list took 32 cache lines per load: 64 uneven sets of
+// 96 dimensions, 32 entries 545 -> 504 us a tree, 500,000 points 119 -> 113, 1M
+// points with 16 entries 73 -> 68.  With 32 entries the duplicate search and the
+// networks, 2,900 half-rate instructions a point, bound it; with 16, HBM.
+constexpr int kFoldThreads = 128;
 template <int KP>
-__global__ void __launch_bounds__(256) k_fold_lists(const float *__restrict__ tree_dist,
-                                                    const int32_t *__restrict__ tree_idx,
-                                                    int64_t n, float *__restrict__ run_dist,
-                                                    int32_t *__restrict__ run_idx) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const int64_t o = p * KP;
+__global__ void __launch_bounds__(kFoldThreads) k_fold_lists(const float *__restrict__ tree_dist,
+                                                             const int32_t *__restrict__ tree_idx,
+                                                             int64_t n,
+                                                             float *__restrict__ run_dist,
+                                                             int32_t *__restrict__ run_idx) {
+  constexpr int Q = KP / 4;  // 16-byte pieces of a list
+  __shared__ uint4 turn[kFoldThreads / 32][32 * Q];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t p0 = (int64_t)blockIdx.x * kFoldThreads + 32 * warp;
+  if (p0 >= n) return;  // the whole warp
+  const int pieces = (int)min64(32, n - p0) * Q;
+  uint4 *buf = turn[warp];
+  const auto slot = [](int p, int c) { return p * Q + (c ^ (Q == 8 ? p & 7 : (p >> 1) & 3)); };
+  const auto fetch = [&](const void *list, bool last_use, uint4 *v) {
+    const uint4 *src = static_cast<const uint4 *>(list) + p0 * Q;
+#pragma unroll
+    for (int i = 0; i < Q; ++i)
+      if (32 * i + lane < pieces) {
+        if (last_use) v[i] = __ldcs(src + 32 * i + lane);
+        else v[i] = src[32 * i + lane];
+      }
+  };
+  const auto to_lists = [&](uint4 *v) {
+#pragma unroll
+    for (int i = 0; i < Q; ++i) buf[slot((32 * i + lane) / Q, lane % Q)] = v[i];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < Q; ++i) v[i] = buf[slot(lane, i)];
+    __syncwarp();
+  };
+  const auto put = [&](const uint4 *v, void *list) {
+    uint4 *dst = static_cast<uint4 *>(list) + p0 * Q;
+#pragma unroll
+    for (int i = 0; i < Q; ++i) buf[slot(lane, i)] = v[i];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < Q; ++i)
+      if (32 * i + lane < pieces) dst[32 * i + lane] = buf[slot((32 * i + lane) / Q, lane % Q)];
+    __syncwarp();
+  };
+  uint4 w[4][Q];  // lanes past the last point fold what lies there and write nothing
+  fetch(tree_dist, true, w[0]);
+  fetch(tree_idx, true, w[1]);
+  fetch(run_dist, false, w[2]);
+  fetch(run_idx, false, w[3]);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) to_lists(w[a]);
   float rd[KP], od[KP];
   int32_t ri[KP], oi[KP];
 #pragma unroll
   for (int j = 0; j < KP; j += 4) {
-    const float4 a = __ldcs(reinterpret_cast<const float4 *>(tree_dist + o) + j / 4);
-    const int4 b = __ldcs(reinterpret_cast<const int4 *>(tree_idx + o) + j / 4);
-    const float4 c = reinterpret_cast<const float4 *>(run_dist + o)[j / 4];
-    const int4 e = reinterpret_cast<const int4 *>(run_idx + o)[j / 4];
-    rd[j] = a.x; rd[j + 1] = a.y; rd[j + 2] = a.z; rd[j + 3] = a.w;
+    const uint4 a = w[0][j / 4], b = w[1][j / 4], c = w[2][j / 4], e = w[3][j / 4];
+    rd[j] = __uint_as_float(a.x); rd[j + 1] = __uint_as_float(a.y);
+    rd[j + 2] = __uint_as_float(a.z); rd[j + 3] = __uint_as_float(a.w);
     ri[j] = b.x; ri[j + 1] = b.y; ri[j + 2] = b.z; ri[j + 3] = b.w;
-    od[j] = c.x; od[j + 1] = c.y; od[j + 2] = c.z; od[j + 3] = c.w;
+    od[j] = __uint_as_float(c.x); od[j + 1] = __uint_as_float(c.y);
+    od[j + 2] = __uint_as_float(c.z); od[j + 3] = __uint_as_float(c.w);
     oi[j] = e.x; oi[j + 1] = e.y; oi[j + 2] = e.z; oi[j + 3] = e.w;
   }
 #pragma unroll
@@ -1050,9 +1099,12 @@ __global__ void __launch_bounds__(256) k_fold_lists(const float *__restrict__ tr
   bitonic_merge_into<KP, KP>(od, oi, rd, ri);
 #pragma unroll
   for (int j = 0; j < KP; j += 4) {
-    reinterpret_cast<float4 *>(run_dist + o)[j / 4] = make_float4(od[j], od[j + 1], od[j + 2], od[j + 3]);
-    reinterpret_cast<int4 *>(run_idx + o)[j / 4] = make_int4(oi[j], oi[j + 1], oi[j + 2], oi[j + 3]);
+    w[0][j / 4] = make_uint4(__float_as_uint(od[j]), __float_as_uint(od[j + 1]),
+                             __float_as_uint(od[j + 2]), __float_as_uint(od[j + 3]));
+    w[1][j / 4] = make_uint4(oi[j], oi[j + 1], oi[j + 2], oi[j + 3]);
   }
+  put(w[0], run_dist);
+  put(w[1], run_idx);
 }
 
 // The same with KP lanes per point, the lists' entries one per lane: the same
@@ -1478,10 +1530,11 @@ drpt_status launch_fold_lists(const MixedTreeArgs &a, cudaStream_t s) {
     return DRPT_ERR_UNSUPPORTED;
   }
   const bool lanes = a.n * a.kp <= kFoldLanes;
-  const unsigned grid = (unsigned)ceil_div(lanes ? a.n * a.kp : a.n, 256);
+  const int threads = lanes ? 256 : kFoldThreads;
+  const unsigned grid = (unsigned)ceil_div(lanes ? a.n * a.kp : a.n, threads);
   auto kern = a.kp == 16 ? (lanes ? k_fold_lanes<16> : k_fold_lists<16>)
                          : (lanes ? k_fold_lanes<32> : k_fold_lists<32>);
-  kern<<<grid, 256, 0, s>>>(a.tree_dist, a.tree_idx, a.n, a.cand_dist, a.cand_idx);
+  kern<<<grid, threads, 0, s>>>(a.tree_dist, a.tree_idx, a.n, a.cand_dist, a.cand_idx);
   DRPT_LAUNCH_CHECK();
   return DRPT_OK;
 }
