@@ -867,12 +867,12 @@ drpt_status learn_and_project(drpt_ctx *c, const void *X, int dtype, int64_t n, 
     const int last = levels - 2;
     const int64_t Gmax = (int64_t)T << last, Umax = tree_level_max_units(S, T, last);
     lv.max_nodes = Gmax;
-  lv.max_units = Umax;
-  DRPT_TRY(ws_get(c, "ls_node_ubase", 2 * Gmax, &lv.node_ubase));
+    lv.max_units = Umax;
+    DRPT_TRY(ws_get(c, "ls_node_ubase", 2 * Gmax, &lv.node_ubase));
     DRPT_TRY(ws_get(c, "ls_unit_node", 2 * Umax, &lv.unit_node));
     DRPT_TRY(ws_get(c, "ls_unit_lo", 2 * Umax, &lv.unit_lo));
     DRPT_TRY(ws_get(c, "ls_n_units", 2 * T, &lv.n_units));
-  DRPT_TRY(ws_get(c, "ls_tickets", Gmax, &lv.tickets));
+    DRPT_TRY(ws_get(c, "ls_tickets", Gmax, &lv.tickets));
     DRPT_TRY(ws_get(c, "ls_node_D", Gmax * kBins, &lv.node_D));
     DRPT_TRY(ws_get(c, "ls_unit_s", 2 * Umax, &lv.unit_s));
     DRPT_TRY(ws_get(c, "ls_unit_hist", Umax * kBins, &lv.unit_hist));

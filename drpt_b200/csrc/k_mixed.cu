@@ -61,8 +61,8 @@ constexpr int kTM = 128;            // rows per tile (M)
 // where those tiles fetch 24.  An MMA of 64 columns also takes 48 cycles for
 // 32 cycles of work (it reads 6 KB of shared memory at 128 bytes per cycle);
 // of 128 or more it runs at its full rate.  Leaf kernels of the 60,000 x 784
-// u8 build (12 trees, 13 K blocks) 2.76 -> 1.37 ms, of 500,000 x 960 in E4M3
-// (32 trees, 8 K blocks) 49.9 -> 38 ms.  The line between 2 and 3: a build
+// u8 build (12 trees, 13 K blocks) 2.76 -> 1.32 ms, of 500,000 x 960 in E4M3
+// (32 trees, 8 K blocks) 49.9 -> 35.3 ms.  The line between 2 and 3: a build
 // with 8 K blocks takes 2.47 ms in shape 2 and 2.65 in shape 3, with 11 blocks
 // 2.52 and 2.54, with 15 blocks 4.32 and 4.11 (one CTA's four epilogue warps
 // are too few for short rows).  Measured slower: A resident on one CTA per SM

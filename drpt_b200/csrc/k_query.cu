@@ -12,7 +12,8 @@
 //                 id): k_query_few reads a leaf for each query, k_query_tile
 //                 once for all queries that fall in it
 //   Q3            the trees' lists merged (a point found in several trees
-//                 counts once): k_query_join, or the builds' cross-tree merge
+//                 counts once): by the query's last block of k_query_few, or
+//                 the builds' cross-tree merge
 #include <algorithm>
 #include <type_traits>
 
