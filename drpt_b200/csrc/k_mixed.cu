@@ -54,7 +54,8 @@ constexpr int kTM = 128;            // rows per tile (M)
 //      The epilogue bounds it, so the warps per SM count.
 //   1: kb <= 4 and 16 keys, A resident (64 KB), 64 columns, 2 CTAs per SM.
 //   2: a stage holds a K block of A too, 128 columns, 2 CTAs per SM.
-//   3: kb >= kWideKb, as 2 with 256 columns, 1 CTA per SM.
+//   3: as 2 with 256 columns, 1 CTA per SM (wide rows, or fairly wide rows and
+//      large leaves: wide_rows).
 // Past shape 0 the feed from L2 bounds the kernel (64-column tiles with A
 // streamed took in 48 bytes per cycle and SM, of the 64 there are): per 64
 // columns and K block shape 1 fetches 8 KB, shape 2 16 KB, shape 3 12 KB,
@@ -62,13 +63,20 @@ constexpr int kTM = 128;            // rows per tile (M)
 // 32 cycles of work (it reads 6 KB of shared memory at 128 bytes per cycle);
 // of 128 or more it runs at its full rate.  Leaf kernels of the 60,000 x 784
 // u8 build (12 trees, 13 K blocks) 2.76 -> 1.32 ms, of 500,000 x 960 in E4M3
-// (32 trees, 8 K blocks) 49.9 -> 35.3 ms.  The line between 2 and 3: a build
-// with 8 K blocks takes 2.47 ms in shape 2 and 2.65 in shape 3, with 11 blocks
-// 2.52 and 2.54, with 15 blocks 4.32 and 4.11 (one CTA's four epilogue warps
-// are too few for short rows).  Measured slower: A resident on one CTA per SM
-// with 128 columns (8 blocks: 71.7 ms per E4M3 build against 65.6 streamed),
-// and A in Tensor Memory (such an MMA takes about 150 cycles at 64 columns).
+// (32 trees, 8 K blocks) 49.9 -> 33.5 ms.  The line between 2 and 3 (one CTA's
+// four epilogue warps are too few for short rows and small leaves, where a
+// larger part of the scores is kept): builds of 200,000 points in leaves of
+// about 780 with 8 K blocks take 2.92 ms in shape 2 and 3.07 in shape 3, with 11
+// 4.04 both, 60,000 x 784 (13 blocks) 3.15 and 2.64.  Leaves of 1,950 with 8
+// blocks 5.12 and 5.08 (16 entries) or 6.40 and 6.31 (32), with 10 blocks 4.99 and
+// 4.74 or 5.92 and 5.82, with 6 3.22 and 3.39; 500,000 x 960 in E4M3 62.6 and 60.6.
+// Measured slower: A resident on one CTA per SM with 128 columns (8 blocks: 71.7
+// ms per E4M3 build against 65.6 streamed), and A in Tensor Memory (such an MMA
+// takes about 150 cycles at 64 columns).
 constexpr int kWideKb = 12;
+bool wide_rows(int kb, int64_t leaf) {
+  return kb >= kWideKb || (kb >= 8 && kb * leaf >= 15000);
+}
 template <int KP, int SHAPE>
 struct MmaCfg {
   static constexpr int tn = SHAPE <= 1 ? 64 : (SHAPE == 2 ? 128 : 256);
@@ -1453,8 +1461,8 @@ drpt_status mma_shaped(const MixedTreeArgs &a, const CUtensorMap &tmA, int kb, c
   if (kb <= 2) return mma_t<KP, 0, FP8>(a, tmA, kb, s);
   if constexpr (KP == 16)
     if (kb <= 4) return mma_t<KP, 1, FP8>(a, tmA, kb, s);
-  if (kb < kWideKb) return mma_t<KP, 2, FP8>(a, tmA, kb, s);
-  return mma_t<KP, 3, FP8>(a, tmA, kb, s);
+  if (wide_rows(kb, a.n / a.nleaf)) return mma_t<KP, 3, FP8>(a, tmA, kb, s);
+  return mma_t<KP, 2, FP8>(a, tmA, kb, s);
 }
 
 template <int KP>
