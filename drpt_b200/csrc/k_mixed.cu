@@ -63,7 +63,7 @@ constexpr int kTM = 128;            // rows per tile (M)
 // 32 cycles of work (it reads 6 KB of shared memory at 128 bytes per cycle);
 // of 128 or more it runs at its full rate.  Leaf kernels of the 60,000 x 784
 // u8 build (12 trees, 13 K blocks) 2.76 -> 1.32 ms, of 500,000 x 960 in E4M3
-// (32 trees, 8 K blocks) 49.9 -> 33.5 ms.  The line between 2 and 3 (one CTA's
+// (32 trees, 8 K blocks) 49.9 -> 33.3 ms.  The line between 2 and 3 (one CTA's
 // four epilogue warps are too few for short rows and small leaves, where a
 // larger part of the scores is kept): builds of 200,000 points in leaves of
 // about 780 with 8 K blocks take 2.92 ms in shape 2 and 3.07 in shape 3, with 11
