@@ -26,8 +26,11 @@
 
 namespace {
 
-// Builds may need up to kBuildBytes besides the unit tables of the next level
-// and the tickets (16 bytes a node and 8 a unit, next to at least 76 and 96).
+// A build may take up to kBuildBytes, counted with the unit tables of one level
+// and without tickets (carve's `planned` false).  The next level's tables and the
+// tickets come on top: 8 bytes a node, a unit and a tree, where each node has at
+// least 76 bytes, each unit 96, and a tree of G nodes at least G + 1 units.  Most
+// of all with one node a tree: 32 bytes on top of 268, 7.6 MiB of 64.
 constexpr size_t kBuildBytes = size_t(64) << 20;
 constexpr size_t kStaticScratchBytes = size_t(72) << 20;  // 72 MiB per device
 constexpr int kMaxDevices = 64;
@@ -87,10 +90,10 @@ struct Layout {
   float *val[2];      // T x n each: split values of the next level
   int32_t *off_tmp;   // T x (nleaf + 1): the side that is not `offsets`
   TreeLevelArgs lv;   // per-level scratch, sized for the deepest level
-  size_t tables;      // bytes of the second unit tables and the tickets
 };
 
-size_t carve(unsigned char *base, int64_t n, int T, int gd, Layout *L) {
+// The bytes taken.  `planned`: with the tables that let a level plan the next.
+size_t carve(unsigned char *base, int64_t n, int T, int gd, Layout *L, bool planned = true) {
   Carver c{base};
   const int nleaf = 1 << (gd - 1);
   const bool deep = gd >= 3;  // two or more levels: intermediates exist
@@ -104,12 +107,11 @@ size_t carve(unsigned char *base, int64_t n, int T, int gd, Layout *L) {
   TreeLevelArgs &a = L->lv;
   a.max_nodes = G;
   a.max_units = U;
-  a.node_ubase = c.take<int32_t>(2 * G);
-  a.unit_node = c.take<int32_t>(2 * U);
-  a.unit_lo = c.take<int32_t>(2 * U);
-  a.n_units = c.take<int32_t>(2 * T);
-  a.tickets = c.take<unsigned>(G);
-  L->tables = 4 * (2 * (size_t)G + 2 * (size_t)U + 2 * (size_t)T);
+  a.node_ubase = c.take<int32_t>(planned ? 2 * G : G + 1);
+  a.unit_node = c.take<int32_t>(planned ? 2 * U : U);
+  a.unit_lo = c.take<int32_t>(planned ? 2 * U : U);
+  a.n_units = c.take<int32_t>(planned ? 2 * T : 1);
+  if (planned) a.tickets = c.take<unsigned>(G);
   a.node_D = c.take<float>(G * kBins);
   a.unit_s = c.take<double>(2 * U);
   a.unit_hist = c.take<unsigned>(U * kBins);
@@ -155,11 +157,11 @@ extern "C" drpt_status drpt_global_trees_noalloc(const float *P, int64_t n, int3
     return DRPT_OK;
   }
   Layout L{};
-  const size_t need = carve(nullptr, n, T, gd, &L);
-  if (need - L.tables > kBuildBytes || need > kStaticScratchBytes) {
-    set_error("drpt_global_trees_noalloc: n=%lld, T=%d, gd=%d needs %zu bytes of scratch; the "
-              "static scratch holds %zu (use drpt_global_trees for this size)",
-              (long long)n, T, gd, need, kStaticScratchBytes);
+  const size_t need = carve(nullptr, n, T, gd, &L, /*planned=*/false);
+  if (need > kBuildBytes || carve(nullptr, n, T, gd, &L) > kStaticScratchBytes) {
+    set_error("drpt_global_trees_noalloc: n=%lld, T=%d, gd=%d needs %zu bytes; a build gets %zu "
+              "of the static scratch (use drpt_global_trees for this size)",
+              (long long)n, T, gd, need, kBuildBytes);
     return DRPT_ERR_INVALID_ARG;
   }
   unsigned char *base = nullptr;

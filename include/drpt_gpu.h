@@ -348,10 +348,11 @@ drpt_status drpt_merge_candidates(drpt_ctx *ctx, const int32_t *cand_idx, const 
  *
  * Scratch comes from a 72 MiB array that is part of the library's device
  * image (every GPU that loads the library holds it until exit); `order` and
- * `offsets` double as one side of the level ping-pong.  A build needs about
- * 12*T*n bytes plus per-level tables; larger builds are rejected with
- * DRPT_ERR_INVALID_ARG and a message naming the bytes needed (T*n up to
- * about 5 million).  The first call on a device looks up the array's device
+ * `offsets` double as one side of the level ping-pong.  A build may take 64 MiB
+ * of it: about 12*T*n bytes plus per-level tables (the rest serves the tables
+ * that plan the next level).  Larger builds are rejected with
+ * DRPT_ERR_INVALID_ARG and a message naming the bytes needed and that limit
+ * (T*n up to about 5 million).  The first call on a device looks up the array's device
  * address (cudaGetSymbolAddress); make that first call before any stream
  * capture.  Every call shares the array: calls whose kernels overlap on the
  * GPU (other streams, other host threads) race and must be serialised. */
