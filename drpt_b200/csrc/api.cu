@@ -65,10 +65,10 @@ struct drpt_index {
   int max_leaf = 0;
   __nv_bfloat16 *w1b = nullptr;
   float *b1 = nullptr, *w2 = nullptr, *b2 = nullptr, *c = nullptr, *inv_sigma = nullptr;
-  // query scratch, one allocation grown on demand; tickets that are 0 between
-  // queries
+  // query scratch for blocks of up to `cap` queries, one allocation grown on
+  // demand; tickets that are 0 between queries
   uint8_t *scratch = nullptr;
-  size_t scratch_bytes = 0;
+  int64_t cap = 0;
   unsigned *tickets = nullptr;
 };
 
@@ -2058,70 +2058,81 @@ drpt_status drpt_index_build(drpt_ctx *c, const drpt_build_desc *desc, const voi
 
 void drpt_index_destroy(drpt_index *index) { index_free(index); }
 
-// Entries of the candidate lists held at a time (8 bytes each: 512 MiB).
+// A call goes block by block; the candidate lists of one hold at most this many
+// entries (8 bytes each: 512 MiB) at the largest k.
 static constexpr int64_t kQueryEntries = (int64_t)64 << 20;
+static constexpr int kQueryK = 32;
+
+// Where the buffers of a block of queries lie in the scratch (256-byte aligned
+// parts), and its bytes.  Their sizes depend on `cap` alone: a block of up to as
+// many queries finds room whatever its k, its rows' alignment and the memory they
+// come from, so a call allocates only when it brings more queries than any before.
+struct QueryScratch {
+  size_t err, P, leaf, ci, cd, cnt, off, items, n_items, rank, list, qi, qd, qx, qxb, total = 0;
+  QueryScratch(const drpt_index *x, int64_t cap) {
+    const size_t esz = x->dtype == DRPT_DTYPE_U8 ? 1 : 4, cols = (size_t)x->T * (x->gd - 1);
+    const QueryRoom r = query_room(cap, x->T, x->nleaf, kQueryK);
+    const size_t pairs = (size_t)cap * x->T;
+    auto part = [&](size_t bytes) {
+      const size_t at = total;
+      total += (bytes + 255) & ~(size_t)255;
+      return at;
+    };
+    err = part(4);
+    P = part(cols * cap * 4);
+    leaf = part(pairs * 4);
+    ci = part((size_t)r.entries * 4);
+    cd = part((size_t)r.entries * 4);
+    cnt = part((size_t)r.buckets * 4);
+    off = part((size_t)r.buckets * 4);
+    items = part((size_t)r.items * sizeof(int4));
+    n_items = part(4);
+    rank = part(r.buckets ? pairs * 4 : 0);
+    list = part(r.buckets ? pairs * 4 : 0);
+    qi = part((size_t)cap * kQueryK * 4);
+    qd = part((size_t)cap * kQueryK * 4);
+    qx = part((size_t)cap * x->d * esz);
+    qxb = part(x->Tl > 0 ? (size_t)cap * x->d_pad * 2 : 0);
+  }
+};
 
 // One block of queries, stream-ordered.  `first`: clears the error flag of the
 // inference kernel, which later blocks of the call add to.
-static drpt_status query_block(drpt_index *x, const void *queries, int64_t nq, int k,
-                               int on_device, bool first, int32_t *out_idx, float *out_dist,
-                               int **err_out, cudaStream_t s) {
-  const int d = x->d, T = x->T, cols = T * (x->gd - 1);
-  const size_t esz = x->dtype == DRPT_DTYPE_U8 ? 1 : 4, pairs = (size_t)nq * T;
+static drpt_status query_block(drpt_index *x, const QueryScratch &l, const void *queries,
+                               int64_t nq, int k, int on_device, bool first, int32_t *out_idx,
+                               float *out_dist, cudaStream_t s) {
+  const int d = x->d, T = x->T;
+  const size_t esz = x->dtype == DRPT_DTYPE_U8 ? 1 : 4;
   const bool aligned = !on_device || (uintptr_t)queries % (4 * esz) == 0;
   const QueryPlan p = query_plan(nq, T, x->nleaf, x->max_leaf, k, aligned, x->Tl == 0);
-  // the block's buffers, laid out in one allocation (16-byte aligned parts)
-  size_t total = 0;
-  auto part = [&](size_t bytes) {
-    const size_t at = total;
-    total += (bytes + 255) & ~(size_t)255;
-    return at;
-  };
-  const size_t o_err = part(4), o_P = part((size_t)cols * nq * 4), o_leaf = part(pairs * 4);
-  const size_t o_ci = part((size_t)p.entries * 4), o_cd = part((size_t)p.entries * 4);
-  const size_t o_cnt = part((size_t)p.buckets * 4), o_off = part((size_t)p.buckets * 4);
-  const size_t o_items = part((size_t)p.items * sizeof(int4)), o_nit = part(4);
-  const size_t o_rank = part(p.qt ? pairs * 4 : 0), o_list = part(p.qt ? pairs * 4 : 0);
-  const size_t o_qi = part(on_device ? 0 : (size_t)nq * k * 4);
-  const size_t o_qd = part(on_device && out_dist ? 0 : (size_t)nq * k * 4);
-  const size_t o_qx = part(on_device ? 0 : (size_t)nq * d * esz);
-  const size_t o_qxb = part(x->Tl > 0 ? (size_t)nq * x->d_pad * 2 : 0);
-  if (total > x->scratch_bytes) {
-    if (x->scratch) DRPT_CUDA(cudaFree(x->scratch));
-    x->scratch = nullptr;
-    x->scratch_bytes = 0;
-    DRPT_CUDA(cudaMalloc((void **)&x->scratch, total));
-    x->scratch_bytes = total;
-  }
   uint8_t *b = x->scratch;
   const void *Q = queries;
   if (!on_device) {
-    DRPT_CUDA(cudaMemcpyAsync(b + o_qx, queries, (size_t)nq * d * esz, cudaMemcpyHostToDevice, s));
-    Q = b + o_qx;
+    DRPT_CUDA(cudaMemcpyAsync(b + l.qx, queries, (size_t)nq * d * esz, cudaMemcpyHostToDevice, s));
+    Q = b + l.qx;
   }
   // the queries' split values: random columns, then the learned MLP outputs
-  float *P = (float *)(b + o_P);
+  float *P = (float *)(b + l.P);
   const CscDev csc{x->csc_col, x->csc_row, x->csc_val, x->ncols_r};
   if (x->ncols_r > 0 && !p.descend) DRPT_TRY(launch_project(Q, x->dtype, nq, d, csc, P, s));
   if (x->Tl > 0) {
-    int *err = (int *)(b + o_err);
-    __nv_bfloat16 *xb = (__nv_bfloat16 *)(b + o_qxb);
+    int *err = (int *)(b + l.err);
+    __nv_bfloat16 *xb = (__nv_bfloat16 *)(b + l.qxb);
     if (first) DRPT_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
     DRPT_TRY(launch_standardise(Q, x->dtype, nq, d, x->d_pad, nullptr, x->c, x->inv_sigma, xb,
                                 nullptr, s));
     DRPT_TRY(launch_mlp_infer(xb, nq, x->d_pad, x->w1b, x->Tl * (x->gd - 1), x->b1, x->w2, x->b2,
                               P + (int64_t)x->ncols_r * nq, err, s));
-    *err_out = err;
   }
-  int32_t *leaf = (int32_t *)(b + o_leaf);
+  int32_t *leaf = (int32_t *)(b + l.leaf);
   if (!p.descend) DRPT_TRY(launch_descend(P, nq, T, x->gd, x->medians, leaf, s));
-  int32_t *oi = on_device ? out_idx : (int32_t *)(b + o_qi);
-  float *od = on_device && out_dist ? out_dist : (float *)(b + o_qd);
+  int32_t *oi = on_device ? out_idx : (int32_t *)(b + l.qi);
+  float *od = on_device && out_dist ? out_dist : (float *)(b + l.qd);
   const QueryArgs a{x->X, x->dtype, d, x->n, Q, nq, T, x->order, x->goff, x->nleaf, leaf, csc,
                     x->medians, x->gd, x->tickets, k,
-                    (int32_t *)(b + o_ci), (float *)(b + o_cd), (int32_t *)(b + o_rank),
-                    (int32_t *)(b + o_cnt), (int32_t *)(b + o_off), (int4 *)(b + o_items),
-                    (int32_t *)(b + o_nit), (int32_t *)(b + o_list), oi, od};
+                    (int32_t *)(b + l.ci), (float *)(b + l.cd), (int32_t *)(b + l.rank),
+                    (int32_t *)(b + l.cnt), (int32_t *)(b + l.off), (int4 *)(b + l.items),
+                    (int32_t *)(b + l.n_items), (int32_t *)(b + l.list), oi, od};
   DRPT_TRY(launch_query(a, p, s));
   if (!on_device) {
     DRPT_CUDA(cudaMemcpyAsync(out_idx, oi, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, s));
@@ -2134,23 +2145,30 @@ static drpt_status query_block(drpt_index *x, const void *queries, int64_t nq, i
 drpt_status drpt_index_query(drpt_index *x, const void *queries, int64_t nq, int32_t k,
                              int32_t on_device, int32_t *out_idx, float *out_dist, void *stream) {
   if (!x || !queries || !out_idx || nq <= 0 || k <= 0) return DRPT_ERR_INVALID_ARG;
-  if (k > 32) {
-    set_error("queries return at most 32 neighbours (k = %d)", k);
+  if (k > kQueryK) {
+    set_error("queries return at most %d neighbours (k = %d)", kQueryK, k);
     return DRPT_ERR_UNSUPPORTED;
   }
   DRPT_CUDA(cudaSetDevice(x->device));
   cudaStream_t s = (cudaStream_t)stream;
-  // blocks of queries whose candidate lists stay within kQueryEntries
-  const int64_t most = std::max<int64_t>(1, kQueryEntries / ((int64_t)x->T * k));
+  const int64_t block = std::max<int64_t>(1, kQueryEntries / ((int64_t)x->T * kQueryK));
+  const int64_t cap = std::min(nq, block);
+  if (cap > x->cap) {
+    if (x->scratch) DRPT_CUDA(cudaFree(x->scratch));
+    x->scratch = nullptr;
+    x->cap = 0;
+    DRPT_CUDA(cudaMalloc((void **)&x->scratch, QueryScratch(x, cap).total));
+    x->cap = cap;
+  }
+  const QueryScratch l(x, x->cap);
   const size_t esz = x->dtype == DRPT_DTYPE_U8 ? 1 : 4;
-  int *err = nullptr;
-  for (int64_t q0 = 0; q0 < nq; q0 += most)
-    DRPT_TRY(query_block(x, static_cast<const uint8_t *>(queries) + (size_t)q0 * x->d * esz,
-                         std::min(most, nq - q0), k, on_device, q0 == 0, out_idx + q0 * k,
-                         out_dist ? out_dist + q0 * k : nullptr, &err, s));
+  for (int64_t q0 = 0; q0 < nq; q0 += block)
+    DRPT_TRY(query_block(x, l, static_cast<const uint8_t *>(queries) + (size_t)q0 * x->d * esz,
+                         std::min(block, nq - q0), k, on_device, q0 == 0, out_idx + q0 * k,
+                         out_dist ? out_dist + q0 * k : nullptr, s));
   if (x->Tl > 0) {
     int herr = 0;
-    DRPT_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    DRPT_CUDA(cudaMemcpyAsync(&herr, x->scratch + l.err, sizeof(int), cudaMemcpyDeviceToHost, s));
     DRPT_CUDA(cudaStreamSynchronize(s));
     if (herr) {
       set_error("a bounded wait in the split-MLP inference kernel gave up");

@@ -511,11 +511,12 @@ int query_group(int64_t nq, int nleaf) {
 
 // Shares that the few-queries form cuts a leaf into: until the pairs fill the
 // SMs, but no share below the block's 256 members.  (More than one share only
-// below 8 * 148 pairs, so below kQueryTickets queries.)
-static_assert(kQueryTickets >= 8 * 148, "lists of shares are joined by the last block");
+// below kMostShares pairs, so below kQueryTickets queries.)
+constexpr int64_t kMostShares = 8 * 148;
+static_assert(kQueryTickets >= kMostShares, "lists of shares are joined by the last block");
 int query_shares(int64_t pairs, int max_leaf) {
-  const int most = (int)ceil_div(std::max(max_leaf, 1), 32 * kFewWarps);
-  return (int)std::max<int64_t>(1, std::min<int64_t>(most, 8 * 148 / std::max<int64_t>(pairs, 1)));
+  const int64_t most = ceil_div(std::max(max_leaf, 1), 32 * kFewWarps);
+  return (int)std::max<int64_t>(1, std::min(most, kMostShares / std::max<int64_t>(pairs, 1)));
 }
 
 }  // namespace
@@ -550,6 +551,17 @@ QueryPlan query_plan(int64_t nq, int T, int nleaf, int max_leaf, int k, bool ali
   }
   p.entries = p.lists * k;
   return p;
+}
+
+QueryRoom query_room(int64_t cap, int T, int nleaf, int k) {
+  const int64_t pairs = cap * T;
+  QueryRoom r{};
+  r.entries = std::max(pairs, kMostShares) * k;  // a list a pair, or shares of few pairs
+  if (query_group(cap, nleaf) > 0) {             // (else no fewer queries are grouped)
+    r.buckets = (int64_t)T * nleaf;
+    r.items = ceil_div(pairs, 16) + std::min(r.buckets, pairs);
+  }
+  return r;
 }
 
 drpt_status launch_query(const QueryArgs &a, const QueryPlan &p, cudaStream_t s) {

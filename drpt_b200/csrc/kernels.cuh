@@ -194,6 +194,13 @@ constexpr int64_t kQueryTickets = 4096;  // queries with a ticket (QueryArgs::ti
 QueryPlan query_plan(int64_t nq, int T, int nleaf, int max_leaf, int k, bool aligned,
                      bool random_only);
 
+// The most that any plan of up to `cap` queries and k neighbours needs, whatever
+// its rows' alignment.
+struct QueryRoom {
+  int64_t entries, buckets, items;
+};
+QueryRoom query_room(int64_t cap, int T, int nleaf, int k);
+
 struct QueryArgs {
   const void *X;               // n x d indexed rows
   int dtype;

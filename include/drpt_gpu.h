@@ -263,8 +263,9 @@ drpt_status drpt_learn_gradient(drpt_ctx *ctx, const float *Xs, int32_t S, int32
  * at a time per index.  Query calls keep their scratch in the index, so the
  * device work of two query calls on one index must not overlap, whatever
  * the streams they run on: wait for one call's stream before issuing the
- * next call on another stream (a call that grows the scratch frees the old
- * buffers). */
+ * next call on another stream.  A call of more queries than any before it
+ * grows the scratch (and frees the old buffers); no other call allocates, so
+ * it can be captured. */
 typedef struct drpt_index drpt_index;
 drpt_status drpt_index_build(drpt_ctx *ctx, const drpt_build_desc *desc, const void *data,
                              int32_t *out_idx, float *out_dist, drpt_stats *stats,
