@@ -121,16 +121,20 @@ __device__ __forceinline__ void warp_join(float &ld, int32_t &li, float d, int32
 // spread over T * S blocks of eight warps and a lane keeps kBurst 16-byte
 // pieces of its row in flight; a whole leaf per query on one warp took 911 us
 // for one query of 6 trees with 1,024-point leaves.  With `trees` the block
-// also finds its leaf itself, and with `tickets` (one per query, 0 between
-// calls) the query's last block merges its lists into the result: one launch
-// where four took 26 us of the GPU.
+// also finds its leaf itself, and with `tickets` (one per query) the query's last
+// block merges its lists into the result: one launch where four took 26 us of the
+// GPU.  A block lifts its query's ticket to `turn` (the call's, in the upper 32
+// bits) before it joins its warps' lists, which hides it (at the block's start it
+// took 0.3 to 1 us), and then counts itself in the lower bits, by the same thread:
+// nothing that an earlier call left there is counted.
 constexpr int kFewWarps = 8;
 template <typename T>
 __global__ void __launch_bounds__(32 * kFewWarps) k_query_few(
     const T *__restrict__ X, int d, int64_t n, const T *__restrict__ Qx, int T_, int S,
     const int32_t *__restrict__ order, const int32_t *__restrict__ goff, int nleaf,
     const int32_t *__restrict__ leaf, QueryTrees trees, int k, int32_t *ci, float *cd,
-    unsigned *tickets, int32_t *__restrict__ oi, float *__restrict__ od) {
+    unsigned long long *tickets, unsigned long long turn, int32_t *__restrict__ oi,
+    float *__restrict__ od) {
   constexpr int kBurst = 8;
   extern __shared__ __align__(16) float qv[];  // the query's d values
   __shared__ float sd[kFewWarps][32];
@@ -190,6 +194,7 @@ __global__ void __launch_bounds__(32 * kFewWarps) k_query_few(
     }
     warp_take(ld, li, sqrtf(acc), p, k, lane);
   }
+  if (tickets && threadIdx.x == 0) atomicMax(tickets + q, turn);
   sd[warp][lane] = ld;
   si[warp][lane] = li;
   __syncthreads();
@@ -202,13 +207,8 @@ __global__ void __launch_bounds__(32 * kFewWarps) k_query_few(
     if (tickets) {
       __threadfence();
       __syncwarp();
-      unsigned old = 0u;
-      if (lane == 0) old = atomicAdd(tickets + q, 1u);
-      old = __shfl_sync(kFull, old, 0);
-      if (lane == 0) {
-        leaf_sh = old == (unsigned)(T_ * S) - 1u;
-        if (leaf_sh) tickets[q] = 0u;  // for the next call
-      }
+      if (lane == 0) leaf_sh = atomicAdd(tickets + q, 1ull) == turn + (unsigned)(T_ * S) - 1u;
+      __syncwarp();
       __threadfence();
     }
   }
@@ -582,7 +582,7 @@ drpt_status launch_query(const QueryArgs &a, const QueryPlan &p, cudaStream_t s)
       using E = std::remove_const_t<std::remove_pointer_t<decltype(X)>>;
       k_query_few<E><<<(unsigned)p.lists, 32 * kFewWarps, a.d * sizeof(float), s>>>(
           X, a.d, a.n, Q, a.T, p.shares, a.order, a.goff, a.nleaf, a.leaf, trees, a.k, a.ci, a.cd,
-          p.join ? a.tickets : nullptr, a.oi, a.od);
+          p.join ? a.tickets : nullptr, (unsigned long long)a.turn << 32, a.oi, a.od);
     };
     if (u8) few((const uint8_t *)a.X, (const uint8_t *)a.Q);
     else few((const float *)a.X, (const float *)a.Q);

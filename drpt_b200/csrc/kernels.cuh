@@ -215,7 +215,9 @@ struct QueryArgs {
   CscDev csc;                  // the split functions and medians (plan.descend)
   const float *medians;
   int gd;
-  unsigned *tickets;           // kQueryTickets, 0 between calls (plan.join)
+  // plan.join: kQueryTickets counters, below turn << 32 (of an earlier turn, or 0)
+  unsigned long long *tickets;
+  uint32_t turn;
   int k;
   int32_t *ci;                 // plan.entries
   float *cd;
