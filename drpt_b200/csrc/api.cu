@@ -502,8 +502,8 @@ int list_width_of(int req, int nn) {
 // (no staging) instead of BF16 / E4M3 tiles on the tensor cores.
 drpt_status mixed_leaf_phase(drpt_ctx *c, const void *X, int dtype, int64_t n, int d, int T,
                              int nn, int kp, int fp8, const int32_t *order, const int32_t *goff,
-                             int nleaf, int32_t *oi, float *od, bool timed, cudaStream_t s,
-                             bool f32gram = false) {
+                             int nleaf, int64_t leaf_rows, int32_t *oi, float *od, bool timed,
+                             cudaStream_t s, bool f32gram = false) {
   const int d_pad = mixed_d_pad(d, fp8);
   cudaEvent_t *ev = c->ev;
   MixedTreeArgs a{};
@@ -513,6 +513,7 @@ drpt_status mixed_leaf_phase(drpt_ctx *c, const void *X, int dtype, int64_t n, i
   a.d = d;
   a.d_pad = d_pad;
   a.nleaf = nleaf;
+  a.leaf_rows = leaf_rows;
   a.T = T;
   a.kp = kp;
   a.fp8 = fp8;
@@ -833,7 +834,7 @@ drpt_status learn_and_project(drpt_ctx *c, const void *X, int dtype, int64_t n, 
     poff = dpf;
   }
   DRPT_TRY(mixed_leaf_phase(c, xraw, DRPT_DTYPE_F32, S, d, 1, kLearnPairs, 16, 0, pord, poff,
-                            chunks, nbr_d, ndist, false, s));
+                            chunks, S / chunks, nbr_d, ndist, false, s));
   DRPT_TRY(mixed_check(c, s));
   std::vector<int32_t> nbr((size_t)S * kLearnPairs);
   DRPT_CUDA(cudaMemcpy(nbr.data(), nbr_d, nbr.size() * 4, cudaMemcpyDeviceToHost));
@@ -1071,8 +1072,8 @@ drpt_status run_mixed(drpt_ctx *c, const drpt_build_desc *desc, const void *X, i
   DRPT_TRY(global_trees(c, P, n, T, gd, 0, medians, &order, &goff, s));
   DRPT_CUDA(cudaEventRecord(ev[2], s));
 
-  DRPT_TRY(mixed_leaf_phase(c, X, desc->dtype, n, d, T, nn, kp, fp8, order, goff, nleaf, oi, od,
-                            /*timed=*/true, s, f32gram));
+  DRPT_TRY(mixed_leaf_phase(c, X, desc->dtype, n, d, T, nn, kp, fp8, order, goff, nleaf, n / nleaf,
+                            oi, od, /*timed=*/true, s, f32gram));
   if (check) DRPT_TRY(mixed_check(c, s));
   if (keep) {
     // the index keeps its own copies: the workspace is reused by later calls
@@ -1251,6 +1252,7 @@ struct BatchPlan {
   int nsets = 0, l0 = 0, gdm = 0, nleaf = 0, T = 0, nn = 0, d = 0, dtype = 0, fp8 = 0, mode = 0;
   int kp = 16;                   // mixed mode: candidates kept per point and tree
   int64_t n = 0;
+  int64_t leaf_rows = 0;         // mean rows of the datasets' leaves (most of the nleaf are empty)
   int ncols = 0;                 // T * (gdm - 1) projected columns
   CscDev csc{};
   int32_t *root_off = nullptr;   // T x (2^l0 + 1)
@@ -1280,10 +1282,13 @@ drpt_status batch_prepare(drpt_ctx *c, const drpt_batch_desc *desc, const int64_
   bp->n = n;
   std::vector<int> gds(nsets);
   int gdm = 2;  // at least one level runs, even if no dataset splits
+  int64_t leaves = 0;
   for (int i = 0; i < nsets; ++i) {
     DRPT_TRY(leaf_depth(offs[i + 1] - offs[i], desc->leaf_size, &gds[i]));
     gdm = std::max(gdm, gds[i]);
+    leaves += (int64_t)1 << (gds[i] - 1);
   }
+  bp->leaf_rows = n / leaves;
   int l0 = 0;
   while ((1 << l0) < nsets) ++l0;
   bp->l0 = l0;
@@ -1454,7 +1459,7 @@ drpt_status batch_enqueue(drpt_ctx *c, const BatchPlan &bp, const void *X, int32
   if (timed) DRPT_CUDA(cudaEventRecord(c->ev[2], s));
   if (bp.mode == DRPT_MODE_MIXED) {
     DRPT_TRY(mixed_leaf_phase(c, X, bp.dtype, n, bp.d, T, bp.nn, bp.kp, bp.fp8, bp.order, bp.goff,
-                              bp.nleaf, oi, od, timed, s));
+                              bp.nleaf, bp.leaf_rows, oi, od, timed, s));
   } else {
     if (timed) DRPT_CUDA(cudaEventRecord(c->ev[3], s));
     LeafKnnArgs ka{X, bp.dtype, n, bp.d, T, bp.nn, bp.order, bp.goff, bp.nleaf, bp.cidx, bp.cdist};

@@ -1461,7 +1461,7 @@ drpt_status mma_shaped(const MixedTreeArgs &a, const CUtensorMap &tmA, int kb, c
   if (kb <= 2) return mma_t<KP, 0, FP8>(a, tmA, kb, s);
   if constexpr (KP == 16)
     if (kb <= 4) return mma_t<KP, 1, FP8>(a, tmA, kb, s);
-  if (wide_rows(kb, a.n / a.nleaf)) return mma_t<KP, 3, FP8>(a, tmA, kb, s);
+  if (wide_rows(kb, a.leaf_rows)) return mma_t<KP, 3, FP8>(a, tmA, kb, s);
   return mma_t<KP, 2, FP8>(a, tmA, kb, s);
 }
 

@@ -117,6 +117,7 @@ struct MixedTreeArgs {
   const int32_t *order;      // this tree's global-leaf order (n)
   const int32_t *goff;       // this tree's leaf starts (nleaf + 1)
   int nleaf;
+  int64_t leaf_rows;         // mean rows of the leaves in use
   int T, tree, kp;           // trees, this tree, candidates kept per point
   int fp8;                   // 0: BF16 tiles; 1: E4M3 tiles with per-row scales
   void *Xb;                  // n x d_pad centred rows in leaf order (BF16 or E4M3)
