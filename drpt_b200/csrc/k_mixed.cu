@@ -65,18 +65,24 @@ constexpr int kTM = 128;            // rows per tile (M)
 // u8 build (12 trees, 13 K blocks) 2.76 -> 1.32 ms, of 500,000 x 960 in E4M3
 // (32 trees, 8 K blocks) 49.9 -> 33.3 ms.  The line between 2 and 3 (one CTA's
 // four epilogue warps are too few for short rows and small leaves, where a
-// larger part of the scores is kept): builds of 200,000 points in leaves of
-// about 780 with 8 K blocks take 2.92 ms in shape 2 and 3.07 in shape 3, with 11
-// 4.04 both, 60,000 x 784 (13 blocks) 3.15 and 2.64.  Leaves of 1,950 with 8
-// blocks 5.12 and 5.08 (16 entries) or 6.40 and 6.31 (32), with 10 blocks 4.99 and
-// 4.74 or 5.92 and 5.82, with 6 3.22 and 3.39; 500,000 x 960 in E4M3 62.6 and 60.6.
+// larger part of the scores is kept): a K block more is worth more in shape 3 and
+// what it costs besides is a leaf's, so the blocks past the fourth are weighed with
+// the mean leaf.  Whole builds of 128 such leaves, 4 trees, 16 entries (32: the
+// same sign or within 1.1%), shape 2 and 3 in ms:
+//   8 blocks    leaves of 1,000 1.68 1.76, 1,500 2.66 2.65, 1,600 2.92 2.97,
+//               1,750 3.37 3.33, 1,900 3.72 3.74
+//   9 blocks    1,000 2.03 2.08, 1,250 2.58 2.57, 1,390 2.90 2.91, 1,450 3.11 3.06,
+//               1,500 3.24 3.16
+//   10 blocks   780 1.66 1.69, 1,000 2.15 2.14, 1,150 2.53 2.50, 1,250 2.75 2.67,
+//               1,500 3.45 3.31
+//   11 blocks   780 1.76 1.77, 1,000 2.28 2.25, 1,200 2.82 2.71, 1,500 3.69 3.50
+//   12 blocks   780 1.85 1.81, 1,500 3.91 3.64
+// and in E4M3 with 8 blocks, leaves of 1,600 3.97 3.99, 1,950 with 32 entries (500,000
+// x 960, 32 trees) 62.6 60.6; with 6 blocks leaves of 1,950 3.22 3.39.
 // Measured slower: A resident on one CTA per SM with 128 columns (8 blocks: 71.7
 // ms per E4M3 build against 65.6 streamed), and A in Tensor Memory (such an MMA
 // takes about 150 cycles at 64 columns).
-constexpr int kWideKb = 12;
-bool wide_rows(int kb, int64_t leaf) {
-  return kb >= kWideKb || (kb >= 8 && kb * leaf >= 15000);
-}
+bool wide_rows(int kb, int64_t leaf) { return kb >= 12 || (kb >= 8 && (kb - 4) * leaf >= 7000); }
 template <int KP, int SHAPE>
 struct MmaCfg {
   static constexpr int tn = SHAPE <= 1 ? 64 : (SHAPE == 2 ? 128 : 256);
