@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(THREADS) k_project(const T *__restrict__ X, in
                                                  CscDev csc, float *__restrict__ P, bool quads,
                                                  bool vec_out) {
   constexpr uint32_t kRow = 4 * PT;                   // bytes of a dimension
+  static_assert(PT >= 8, "quads to exchange");
   constexpr uint32_t kSwap = 16 * (PT >= 32 ? 7 : PT / 4 - 1);  // its quads' exchange
   extern __shared__ __align__(16) uint8_t xs[];  // d x kRow
   // byte at which dimension k has the quad of points that starts at byte q16
@@ -180,19 +181,18 @@ void project_t(const T *X, int64_t n, int d, const CscDev &csc, float *P, int pt
   else if (smem <= kHalfSmem) launch(k_project<T, 32, 256>, 256);
   else if (pts == 32) launch(k_project<T, 32, 1024>, 1024);
   else if (pts == 16) launch(k_project<T, 16, 1024>, 1024);
-  else if (pts == 8) launch(k_project<T, 8, 1024>, 1024);
-  else launch(k_project<T, 4, 1024>, 1024);
+  else launch(k_project<T, 8, 1024>, 1024);
 }
 
 }  // namespace
 
 // 128 or 64 points while two such blocks fit on an SM, then 32 or what one
-// block holds.
+// block holds: 8 at the largest d that launch_project takes.
 int project_points_per_block(int d) {
   for (int pts = 128; pts > 32; pts /= 2)
     if (project_smem(pts, d) <= kHalfSmem) return pts;
   int pts = 32;
-  while (pts > 4 && project_smem(pts, d) > 227 * 1024) pts /= 2;
+  while (pts > 8 && project_smem(pts, d) > 227 * 1024) pts /= 2;
   return pts;
 }
 
