@@ -205,7 +205,7 @@ drpt_status launch_project(const void *X, int dtype, int64_t n, int d, const Csc
   }
   int pts = project_points_per_block(d);
   // few points: smaller blocks, down to 32, until every SM has one
-  while (!csc.blocks && pts > 32 && ceil_div(n, pts) < 148) pts /= 2;
+  while (!csc.blocks && pts > 32 && ceil_div(n, pts) < device_sm_count()) pts /= 2;
   const unsigned grid = csc.blocks ? (unsigned)csc.nblocks : (unsigned)ceil_div(n, pts);
   if (dtype == DRPT_DTYPE_U8)
     project_t(static_cast<const uint8_t *>(X), n, d, csc, P, pts, grid, s);

@@ -510,13 +510,13 @@ int query_group(int64_t nq, int nleaf) {
 }
 
 // Shares that the few-queries form cuts a leaf into: until the pairs fill the
-// SMs, but no share below the block's 256 members.  (More than one share only
-// below kMostShares pairs, so below kQueryTickets queries.)
-constexpr int64_t kMostShares = 8 * 148;
-static_assert(kQueryTickets >= kMostShares, "lists of shares are joined by the last block");
+// SMs, but no share below the block's 256 members.  More than one share only
+// below kQueryTickets pairs (so queries): lists of shares are joined by the last
+// block.
+int64_t most_shares() { return std::min<int64_t>(8 * device_sm_count(), kQueryTickets); }
 int query_shares(int64_t pairs, int max_leaf) {
   const int64_t most = ceil_div(std::max(max_leaf, 1), 32 * kFewWarps);
-  return (int)std::max<int64_t>(1, std::min(most, kMostShares / std::max<int64_t>(pairs, 1)));
+  return (int)std::max<int64_t>(1, std::min(most, most_shares() / std::max<int64_t>(pairs, 1)));
 }
 
 }  // namespace
@@ -556,7 +556,7 @@ QueryPlan query_plan(int64_t nq, int T, int nleaf, int max_leaf, int k, bool ali
 QueryRoom query_room(int64_t cap, int T, int nleaf, int k) {
   const int64_t pairs = cap * T;
   QueryRoom r{};
-  r.entries = std::max(pairs, kMostShares) * k;  // a list a pair, or shares of few pairs
+  r.entries = std::max(pairs, most_shares()) * k;  // a list a pair, or shares of few pairs
   if (query_group(cap, nleaf) > 0) {             // (else no fewer queries are grouped)
     r.buckets = (int64_t)T * nleaf;
     r.items = ceil_div(pairs, 16) + std::min(r.buckets, pairs);
