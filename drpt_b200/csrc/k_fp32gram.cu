@@ -4,8 +4,9 @@
 // cores (packed FP32x2 multiply-adds) instead of BF16 tiles on the tensor
 // cores.  It is the fastest plain FP32 counterpart of the mixed form (the
 // reference's own per-pair subtract / multiply / add sequence, kept bit for
-// bit by k_leaf_knn, takes three FP32 operations per dimension and pair; this
-// takes one).
+// bit by the exact form's kernels, k_leaf_tri, k_leaf_tiles_exact and, above 32
+// neighbours, k_leaf_knn, takes three FP32 operations per dimension and pair;
+// this takes one).
 //
 //   k_row_norms   ||x||^2 of every row in FP32 (once per build)
 //   k_leaf_f32    per CTA one 128-row tile of a global leaf against every

@@ -12,7 +12,11 @@
 //   k_leaf_tri          k <= 32, leaves of up to 128 points: each pair once
 //   k_leaf_tiles_exact  k <= 32, larger leaves (k_fp32gram.cu)
 //   k_leaf_knn          k > 32: 64 x 64 tiles of all pairs, one thread per row
-//                       folding the tile's candidates into its list
+//                       folding the tile's candidates into its list.  (Leaves of
+//                       65 to 128 points in one 128 x 128 tile are slower, fewer
+//                       CTAs fit an SM: 100,000 x 128, 8 trees, leaves of about
+//                       98, 33 neighbours 13.4 ms of leaf kernels, 7.6 so; 64
+//                       neighbours 22.3 and 15.9.)
 //
 // Output: for point p and tree t, cand[(p*T + t)*k + j], j < k, sorted by
 // (distance, index), the point itself excluded; slots beyond the leaf size
@@ -25,15 +29,16 @@ namespace drpt {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kTile = 64;              // k_leaf_knn: rows and columns of a tile
 constexpr int kChunk = 32;             // dimensions staged per step
 constexpr int kLd = kChunk + 1;        // padded row stride in shared memory
 constexpr int kTriThreads = 160;       // k_leaf_tri: threads, dimensions staged per step
 constexpr int kTriKc = 32;
 
-template <int TM, typename T>
+template <typename T>
 __device__ __forceinline__ void stage_rows(float *dst, const T *__restrict__ X, int d,
                                            const int32_t *ids, int rows, int k0) {
-  for (int e = threadIdx.x; e < TM * kChunk; e += kThreads) {
+  for (int e = threadIdx.x; e < kTile * kChunk; e += kThreads) {
     const int r = e / kChunk, kk = e - r * kChunk;
     float v = 0.0f;
     if (r < rows && k0 + kk < d) v = (float)X[(int64_t)ids[r] * d + k0 + kk];
@@ -41,15 +46,14 @@ __device__ __forceinline__ void stage_rows(float *dst, const T *__restrict__ X, 
   }
 }
 
-template <int TM>
 constexpr size_t leaf_smem(int k) {
-  return sizeof(float) * (2 * TM * kLd + TM * (TM + 1)) +
-         (sizeof(float) + sizeof(int32_t)) * TM * (k + 1) + sizeof(int32_t) * 2 * TM;
+  return sizeof(float) * (2 * kTile * kLd + kTile * (kTile + 1)) +
+         (sizeof(float) + sizeof(int32_t)) * kTile * (k + 1) + sizeof(int32_t) * 2 * kTile;
 }
 
-template <int TM, typename T>
+template <typename T>
 __global__ void __launch_bounds__(kThreads) k_leaf_knn(LeafKnnArgs a) {
-  constexpr int MT = TM / 16;
+  constexpr int TM = kTile, MT = TM / 16;
   extern __shared__ float smem[];
   float *xr = smem;                          // TM x kLd
   float *xc = xr + TM * kLd;                 // TM x kLd
@@ -87,8 +91,8 @@ __global__ void __launch_bounds__(kThreads) k_leaf_knn(LeafKnnArgs a) {
         for (int j = 0; j < MT; ++j) acc[i][j] = 0.0f;
       const float *xcol = same ? xr : xc;
       for (int k0 = 0; k0 < a.d; k0 += kChunk) {
-        stage_rows<TM>(xr, X, a.d, rid, rows, k0);
-        if (!same) stage_rows<TM>(xc, X, a.d, cid, cols, k0);
+        stage_rows(xr, X, a.d, rid, rows, k0);
+        if (!same) stage_rows(xc, X, a.d, cid, cols, k0);
         __syncthreads();
 #pragma unroll 4
         for (int kk = 0; kk < kChunk; ++kk) {
@@ -316,12 +320,12 @@ drpt_status launch_tris(const LeafKnnArgs &a, unsigned blocks, cudaStream_t s) {
   return launch_tri<T, 128, 4>(a, 96, vec, blocks, s);
 }
 
-template <int TM, typename T>
+template <typename T>
 drpt_status launch_one(const LeafKnnArgs &a, unsigned blocks, cudaStream_t s) {
-  const size_t smem = leaf_smem<TM>(a.k);
-  DRPT_CUDA(cudaFuncSetAttribute(k_leaf_knn<TM, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const size_t smem = leaf_smem(a.k);
+  DRPT_CUDA(cudaFuncSetAttribute(k_leaf_knn<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-  k_leaf_knn<TM, T><<<blocks, kThreads, smem, s>>>(a);
+  k_leaf_knn<T><<<blocks, kThreads, smem, s>>>(a);
   DRPT_LAUNCH_CHECK();
   return DRPT_OK;
 }
@@ -341,8 +345,8 @@ drpt_status launch_leaf_knn_exact(const LeafKnnArgs &a, cudaStream_t s) {
                                       : launch_tris<float>(a, (unsigned)blocks, s));
     return launch_leaf_tiles_exact(a, 128, s);
   }
-  return a.dtype == DRPT_DTYPE_U8 ? launch_one<64, uint8_t>(a, (unsigned)blocks, s)
-                                  : launch_one<64, float>(a, (unsigned)blocks, s);
+  return a.dtype == DRPT_DTYPE_U8 ? launch_one<uint8_t>(a, (unsigned)blocks, s)
+                                  : launch_one<float>(a, (unsigned)blocks, s);
 }
 
 int leaf_knn_exact_kernels(int k) { return k <= 32 ? 4 : 1; }
