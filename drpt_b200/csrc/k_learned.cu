@@ -224,10 +224,11 @@ __global__ void k_point_pairs(const float *__restrict__ f, int S, const int32_t 
   const int n = no[i];
   const float fi = ft[i];
   float lin = 0.0f, sq = 0.0f;
-  // kBurst neighbours' loads in flight; their terms are added in order (13 -> 10
-  // us at 8,192 points, 8 trees, 10 neighbours: the chains of the points with
-  // many in-pairs)
-  constexpr int kBurst = 8;
+  // kBurst neighbours' loads in flight, values only of those in the node; their
+  // terms are added in order (8 trees, 10 neighbours, against one neighbour after
+  // the other: 8,192 points 12.4 -> 9.5 us, the chains of the points with many
+  // in-pairs; 50,000 points 53 -> 51, with all values loaded, eight at a time, 67)
+  constexpr int kBurst = 4;
   const auto terms = [&](const int32_t *idx, int count, auto add) {
     for (int b = 0; b < count; b += kBurst) {
       int j[kBurst], m[kBurst];
@@ -235,13 +236,12 @@ __global__ void k_point_pairs(const float *__restrict__ f, int S, const int32_t 
 #pragma unroll
       for (int q = 0; q < kBurst; ++q) j[q] = b + q < count ? idx[b + q] : -1;
 #pragma unroll
-      for (int q = 0; q < kBurst; ++q) {
-        m[q] = j[q] >= 0 ? no[j[q]] : -1;
-        v[q] = j[q] >= 0 ? ft[j[q]] : 0.0f;
-      }
+      for (int q = 0; q < kBurst; ++q) m[q] = j[q] >= 0 ? no[j[q]] : -1;
+#pragma unroll
+      for (int q = 0; q < kBurst; ++q) v[q] = m[q] == n ? ft[j[q]] : 0.0f;
 #pragma unroll
       for (int q = 0; q < kBurst; ++q)
-        if (j[q] >= 0 && m[q] == n) add(fi - v[q]);
+        if (m[q] == n) add(fi - v[q]);
     }
   };
   terms(nbr + (int64_t)i * k, k, [&](float df) {
