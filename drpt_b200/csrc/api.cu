@@ -2079,7 +2079,7 @@ struct QueryScratch {
   size_t err, P, leaf, ci, cd, cnt, off, items, n_items, rank, list, qi, qd, qx, qxb, total = 0;
   QueryScratch(const drpt_index *x, int64_t cap) {
     const size_t esz = x->dtype == DRPT_DTYPE_U8 ? 1 : 4, cols = (size_t)x->T * (x->gd - 1);
-    const QueryRoom r = query_room(cap, x->T, x->nleaf, kQueryK);
+    const QueryRoom r = query_room(cap, x->T, x->nleaf, x->max_leaf, kQueryK);
     const size_t pairs = (size_t)cap * x->T;
     auto part = [&](size_t bytes) {
       const size_t at = total;

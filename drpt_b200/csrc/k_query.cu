@@ -514,9 +514,10 @@ int query_group(int64_t nq, int nleaf) {
 // below kQueryTickets pairs (so queries): lists of shares are joined by the last
 // block.
 int64_t most_shares() { return std::min<int64_t>(8 * device_sm_count(), kQueryTickets); }
+int64_t leaf_shares(int max_leaf) { return ceil_div(std::max(max_leaf, 1), 32 * kFewWarps); }
 int query_shares(int64_t pairs, int max_leaf) {
-  const int64_t most = ceil_div(std::max(max_leaf, 1), 32 * kFewWarps);
-  return (int)std::max<int64_t>(1, std::min(most, most_shares() / std::max<int64_t>(pairs, 1)));
+  return (int)std::max<int64_t>(
+      1, std::min(leaf_shares(max_leaf), most_shares() / std::max<int64_t>(pairs, 1)));
 }
 
 }  // namespace
@@ -553,11 +554,12 @@ QueryPlan query_plan(int64_t nq, int T, int nleaf, int max_leaf, int k, bool ali
   return p;
 }
 
-QueryRoom query_room(int64_t cap, int T, int nleaf, int k) {
+QueryRoom query_room(int64_t cap, int T, int nleaf, int max_leaf, int k) {
   const int64_t pairs = cap * T;
   QueryRoom r{};
-  r.entries = std::max(pairs, most_shares()) * k;  // a list a pair, or shares of few pairs
-  if (query_group(cap, nleaf) > 0) {             // (else no fewer queries are grouped)
+  // a list a pair, or the shares of few pairs
+  r.entries = std::max(pairs, std::min(pairs * leaf_shares(max_leaf), most_shares())) * k;
+  if (query_group(cap, nleaf) > 0) {  // (else no fewer queries are grouped)
     r.buckets = (int64_t)T * nleaf;
     r.items = ceil_div(pairs, 16) + std::min(r.buckets, pairs);
   }

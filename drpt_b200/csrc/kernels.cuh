@@ -200,7 +200,7 @@ QueryPlan query_plan(int64_t nq, int T, int nleaf, int max_leaf, int k, bool ali
 struct QueryRoom {
   int64_t entries, buckets, items;
 };
-QueryRoom query_room(int64_t cap, int T, int nleaf, int k);
+QueryRoom query_room(int64_t cap, int T, int nleaf, int max_leaf, int k);
 
 struct QueryArgs {
   const void *X;               // n x d indexed rows
