@@ -354,6 +354,10 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_leaf_f32(
 // id) of its lanes' columns, the lists in shared memory between tiles.
 // 100,000 x 128 whole leaves of 1,024 (FP32 leaf form, 4 trees): build 19.5 ->
 // 10.2 ms against 64 x 64 tiles with scalar operations and serial selection.
+// Leaves just above 128 points pay for 256 x 256 pairs: of leaves of 128 on average,
+// half of them above (131,072 points, 8 trees), 32 dimensions and 5 neighbours take
+// 2.7 ms where those tiles took 2.1, 10 neighbours 3.1 and 3.3, 128 dimensions and
+// 10 neighbours 5.8 and 6.2.
 constexpr int kExactThreads = 256, kExactK = 32;
 constexpr size_t kExactSmem =
     sizeof(float) * (kPool + kRows * kExactK) + sizeof(int32_t) * (kRows + kCols + kRows * kExactK);
