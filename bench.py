@@ -748,9 +748,13 @@ def main():
         achieved = flops / (leaf_ms * 1e-3) / 1e12
         sm_mhz = clk.get("sm_mhz") or peaks.get("sm_max_mhz", 1965.0)
         fp32_peak = 148 * 128 * sm_mhz * 1e6 / 1e12
-        roofline = {"kernel": "k_leaf_knn (exact FP32 leaf brute force)", "bound": "fp32",
+        roofline = {"kernel": "k_leaf_tri, k_leaf_tiles_exact (exact FP32 leaf brute force: leaves "
+                              "of up to 128 points and larger): the leaf phase of a build",
+                    "bound": "fp32",
                     "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
-                    "frac": achieved / fp32_peak, "traffic": _traffic_per_launch("k_leaf_knn"),
+                    "frac": achieved / fp32_peak, "traffic": _traffic_per_launch("exact_leaves"),
+                    "traffic_source": "profiles/traffic.json: DRAM bytes of the leaf phase of a "
+                                      "262,144-point build (not measured in this run)",
                     "peak_source": "nominal FP32 issue rate (148 SMs x 128 lanes x median SM "
                                    "clock); MEASURED_PEAKS.json holds no FP32 figure",
                     "algorithmic_flops_per_launch": flops}
