@@ -30,6 +30,7 @@
 // Reference: the leaf brute force MDRPT::calculate_nns (mdrpt.cpp:123-212)
 // with MathOp::calculate_distance (math_operations.cpp:385-396).
 #include "kernels.cuh"
+#include "leaf_lists.cuh"
 #include "sm100.cuh"
 #include "warp_list.cuh"
 
@@ -180,6 +181,8 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_leaf_f32(
   const int r0 = tile.z;
   if (m > kMaxLeaf) {
     if (threadIdx.x == 0) atomicOr(err, 2);
+    empty_lists<KP>(order + lo + r0, min(kRows, m - r0), tree > 0 ? tree_idx : run_idx,
+                    tree > 0 ? tree_dist : run_dist);
     return;
   }
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;

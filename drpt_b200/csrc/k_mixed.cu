@@ -38,6 +38,7 @@
 #include <type_traits>
 
 #include "kernels.cuh"
+#include "leaf_lists.cuh"
 #include "sm100.cuh"
 
 namespace drpt {
@@ -635,6 +636,8 @@ __global__ void __launch_bounds__(MmaCfg<KP, SHAPE>::threads,
   const int r0 = tile.z;
   if (m > kMaxLeaf) {  // the candidate keys address at most kMaxLeaf columns
     if (threadIdx.x == 0) atomicOr(err, 2);
+    empty_lists<KP>(order + lo + r0, min(kTM, m - r0), tree > 0 ? tree_idx : run_idx,
+                    tree > 0 ? tree_dist : run_dist);
     return;  // uniform for the whole block
   }
   const int nct = (m + TN - 1) / TN;
