@@ -1003,7 +1003,9 @@ __global__ void __launch_bounds__(MmaCfg<KP, SHAPE>::threads,
 #pragma unroll
       for (int j = 0; j < KP; ++j) {
         const uint32_t key = __float_as_uint(td[j]);
-        const bool have = key != 0x7f800000u;
+        // (a score of -inf, its column's bits set, is a NaN, of which the networks
+        // make one with all bits set: no column of the leaf)
+        const bool have = key != 0x7f800000u && (int)(key & kColMask) < m;
         const int32_t q = have ? __ldg(order + lo + (int32_t)(key & kColMask)) : -1;
         rd[j] = have ? nr + __uint_as_float(key & ~kColMask) : __int_as_float(0x7f800000);
         ri[j] = q;

@@ -1,7 +1,7 @@
-"""Data that the trees cannot split below the leaf kernels' limit of 8,192 points
-(rows that are all alike, one of NaNs): the build ends with the error that
-names the limit, whatever an earlier build left in the workspace, and the next one
-is right.  Needs a B200."""
+"""Data at the leaf kernels' limits.  Rows that the trees cannot split below 8,192
+points (all alike, one of NaNs): the build ends with the error that names the limit,
+whatever an earlier build left in the workspace, and the next one is right.  Rows so
+far out that their scores overflow: no list names what is no row.  Needs a B200."""
 import numpy as np
 import pytest
 
@@ -42,3 +42,20 @@ def test_leaf_beyond_the_limit(torch, kw, nn, data):
         assert e.value.status == 8
     got = build_graph(big, 3, nn, 5, leaf_size=512, **kw)[:2]
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("kw", [dict(mode="mixed"), dict(mode="mixed", precision="fp8"),
+                                dict(mode="fp32_gram")])
+@pytest.mark.parametrize("nn", [10, 20])
+@pytest.mark.parametrize("d", [64, 104])
+def test_rows_whose_products_overflow(torch, kw, nn, d):
+    # two rows so far out that their products with the others are infinite: their
+    # scores are -inf or NaN.  The other rows' lists are those without them.
+    r = np.random.default_rng(d + nn)
+    X = (r.standard_normal((3_002, d)) * 1e7).astype(np.float32)
+    X[3_000:] = np.where(r.random((2, d)) < 0.5, -1e30, 1e30)
+    X = torch.from_numpy(X).cuda()
+    want = build_graph(X[:3_000].contiguous(), 2, nn, 5, leaf_size=4096, **kw)[:2]
+    idx, dist = build_graph(X, 2, nn, 5, leaf_size=4096, **kw)[:2]
+    assert torch.equal(idx[:3_000], want[0]) and torch.equal(dist[:3_000], want[1])
+    assert ((idx[3_000:] >= -1) & (idx[3_000:] < 3_002)).all()
