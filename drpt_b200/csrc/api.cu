@@ -1339,12 +1339,18 @@ drpt_status batch_prepare(drpt_ctx *c, const drpt_batch_desc *desc, const int64_
       blocks.push_back((int32_t)std::min<int64_t>(pts, offs[i + 1] - r));
       blocks.push_back(set_of_depth[gds[i]]);
     }
+  // tables of the batch: a captured batch's own, which its replays read after
+  // other batches of the context
+  const std::string tag = desc->use_graph ? "bg_" : "bt_";
+  const auto table = [&](const char *name, size_t count, auto **out) {
+    return ws_get(c, (tag + name).c_str(), std::max<size_t>(count, 1), out);
+  };
   int32_t *dcol, *drow, *dblk;
   float *dval;
-  DRPT_TRY(ws_get(c, "bt_colptr", colptr.size(), &dcol));
-  DRPT_TRY(ws_get(c, "bt_row", std::max<size_t>(row.size(), 1), &drow));
-  DRPT_TRY(ws_get(c, "bt_val", std::max<size_t>(val.size(), 1), &dval));
-  DRPT_TRY(ws_get(c, "bt_blocks", std::max<size_t>(blocks.size(), 1), &dblk));
+  DRPT_TRY(table("colptr", colptr.size(), &dcol));
+  DRPT_TRY(table("row", row.size(), &drow));
+  DRPT_TRY(table("val", val.size(), &dval));
+  DRPT_TRY(table("blocks", blocks.size(), &dblk));
   // root slots, stop depths and dataset offsets
   std::vector<int32_t> ro((size_t)T * (nroot + 1));
   for (int t = 0; t < T; ++t)
@@ -1352,9 +1358,9 @@ drpt_status batch_prepare(drpt_ctx *c, const drpt_batch_desc *desc, const int64_
       ro[(size_t)t * (nroot + 1) + j] = (int32_t)offs[std::min(j, nsets)];
   std::vector<int8_t> stop(nroot, 0);
   for (int i = 0; i < nsets; ++i) stop[i] = (int8_t)(gds[i] - 1);
-  DRPT_TRY(ws_get(c, "bt_root_off", ro.size(), &bp->root_off));
-  DRPT_TRY(ws_get(c, "bt_stop", stop.size(), &bp->stop));
-  DRPT_TRY(ws_get(c, "bt_set_off", (size_t)nsets + 1, &bp->set_off));
+  DRPT_TRY(table("root_off", ro.size(), &bp->root_off));
+  DRPT_TRY(table("stop", stop.size(), &bp->stop));
+  DRPT_TRY(table("set_off", (size_t)nsets + 1, &bp->set_off));
   // every other buffer of the build, sized now so that a captured run
   // allocates nothing
   DRPT_TRY(ws_get(c, "P", std::max<size_t>(ncols, 1) * n, &bp->P));
