@@ -219,6 +219,12 @@ drpt_status upload_csc(drpt_ctx *c, const HostCsc &h, const char *tag, CscDev *c
   return DRPT_OK;
 }
 
+// Rows for the whole-leaf forms, which read them in 16-byte (u8: 4-byte) pieces:
+// rows from the host, or that start elsewhere on the device, are copied.
+bool rows_off(const void *data, int dtype) {
+  return (uintptr_t)data % (dtype == DRPT_DTYPE_U8 ? 4 : 16) != 0;
+}
+
 // K1 on a host CSC.
 drpt_status project_cols(drpt_ctx *c, const void *X, int dtype, int64_t n, int d, const HostCsc &h,
                          float *P, cudaStream_t s, const char *tag = "csc") {
@@ -1267,8 +1273,10 @@ struct BatchPlan {
   float *cdist = nullptr;
 };
 
+// `tag` names the tables of the batch: a captured batch's own, which its replays
+// read after other batches of the context.
 drpt_status batch_prepare(drpt_ctx *c, const drpt_batch_desc *desc, const int64_t *offs,
-                          BatchPlan *bp, cudaStream_t s) {
+                          const std::string &tag, BatchPlan *bp, cudaStream_t s) {
   const int nsets = desc->nsets, T = desc->ntrees, d = desc->d;
   const int64_t n = offs[nsets];
   bp->nsets = nsets;
@@ -1339,9 +1347,6 @@ drpt_status batch_prepare(drpt_ctx *c, const drpt_batch_desc *desc, const int64_
       blocks.push_back((int32_t)std::min<int64_t>(pts, offs[i + 1] - r));
       blocks.push_back(set_of_depth[gds[i]]);
     }
-  // tables of the batch: a captured batch's own, which its replays read after
-  // other batches of the context
-  const std::string tag = desc->use_graph ? "bg_" : "bt_";
   const auto table = [&](const char *name, size_t count, auto **out) {
     return ws_get(c, (tag + name).c_str(), std::max<size_t>(count, 1), out);
   };
@@ -1587,10 +1592,14 @@ drpt_status drpt_build_graph_batched(drpt_ctx *c, const drpt_batch_desc *desc,
   cudaEvent_t *ev = c->ev;
   const size_t esz = desc->dtype == DRPT_DTYPE_U8 ? 1 : 4;
   const int launches0 = c->launches;
+  // (rows that are copied first are not captured)
+  const bool off = desc->data_on_device && desc->mode == DRPT_MODE_MIXED &&
+                   rows_off(data, desc->dtype);
+  const bool use_graph = desc->use_graph && !off;
 
   // graph replay
   std::string key;
-  if (desc->use_graph) {
+  if (use_graph) {
     key = batch_key(desc, offsets, data, out_idx, out_dist);
     if (!c->gstream) DRPT_CUDA(cudaStreamCreateWithFlags(&c->gstream, cudaStreamNonBlocking));
     if (c->gexec && c->gkey == key && c->gexec_gen == c->ws_gen) {
@@ -1619,10 +1628,12 @@ drpt_status drpt_build_graph_batched(drpt_ctx *c, const drpt_batch_desc *desc,
 
   DRPT_CUDA(cudaEventRecord(ev[0], s));
   const void *X = data;
-  if (!desc->data_on_device) {
+  if (!desc->data_on_device || off) {
     void *xd;
     DRPT_TRY(ws_get(c, "x", (size_t)n * d * esz, (uint8_t **)&xd));
-    DRPT_CUDA(cudaMemcpyAsync(xd, data, (size_t)n * d * esz, cudaMemcpyHostToDevice, s));
+    DRPT_CUDA(cudaMemcpyAsync(
+        xd, data, (size_t)n * d * esz,
+        desc->data_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
     X = xd;
   }
   int32_t *oi = out_idx;
@@ -1634,7 +1645,7 @@ drpt_status drpt_build_graph_batched(drpt_ctx *c, const drpt_batch_desc *desc,
     DRPT_TRY(ws_get(c, "out_dist", (size_t)n * nn, &od));
   }
   BatchPlan bp;
-  DRPT_TRY(batch_prepare(c, desc, offsets, &bp, s));
+  DRPT_TRY(batch_prepare(c, desc, offsets, use_graph ? "bg_" : "bt_", &bp, s));
   DRPT_CUDA(cudaEventRecord(ev[1], s));
   DRPT_TRY(batch_enqueue(c, bp, X, oi, od, /*timed=*/true, s));
   if (!desc->out_on_device) {
@@ -1660,7 +1671,7 @@ drpt_status drpt_build_graph_batched(drpt_ctx *c, const drpt_batch_desc *desc,
     stats->ms_total = elapsed(ev[0], ev[6]);
     if (desc->mode == DRPT_MODE_MIXED) leaf_phase_ms(c, &stats->ms_leaf_stage, &stats->ms_leaf_mma);
   }
-  if (desc->use_graph) {
+  if (use_graph) {
     // capture the device work of this batch for the next calls (every
     // buffer is sized already, so the captured launches allocate nothing)
     const int l0 = c->launches;
@@ -1771,10 +1782,14 @@ static drpt_status build_graph_impl(drpt_ctx *c, const drpt_build_desc *desc, co
   // Input rows on the device.
   const size_t esz = desc->dtype == DRPT_DTYPE_U8 ? 1 : 4;
   const void *X = data;
-  if (!desc->data_on_device) {
+  const bool whole_leaves = desc->mode == DRPT_MODE_MIXED || desc->mode == DRPT_MODE_FP32_GRAM;
+  if (!desc->data_on_device || (whole_leaves && desc->projection == DRPT_PROJECTION_GAUSSIAN &&
+                                rows_off(data, desc->dtype))) {
     void *xd;
     DRPT_TRY(ws_get(c, "x", (size_t)n * d * esz, (uint8_t **)&xd));
-    DRPT_CUDA(cudaMemcpyAsync(xd, data, (size_t)n * d * esz, cudaMemcpyHostToDevice, s));
+    DRPT_CUDA(cudaMemcpyAsync(
+        xd, data, (size_t)n * d * esz,
+        desc->data_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
     X = xd;
   }
 
